@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(256, 2) segment_kernel(u64 *__restrict__ X, u6
                         else if (sg.kind == SIGN_Z)
                             rd[p] ^= v.x;
                         else
-                            rd[p] ^= s_recw[p * rs + sg.rec] & v.y;
+                            rd[p] ^= s_recw[p * rs + sg.rec] & (sg.kind == SIGN_REC_X ? v.y : v.x);
                     }
                 }
 #pragma unroll
@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(256, 2) segment_kernel(u64 *__restrict__ X, u6
                         else if (sg.kind == SIGN_Z)
                             rd ^= v.x;
                         else
-                            rd ^= s_recw[kk * rs + sg.rec] & v.y;
+                            rd ^= s_recw[kk * rs + sg.rec] & (sg.kind == SIGN_REC_X ? v.y : v.x);
                     }
 #pragma unroll
                     for (int u = 0; u < NE; ++u)
@@ -635,7 +635,7 @@ __global__ void __launch_bounds__(256, 2) segment_kernel(u64 *__restrict__ X, u6
                 for (int it = lane; it < nsg + nent; it += 32) {
                     if (it < nsg) {
                         const SegSign sg = s_signs[it];
-                        const u64 m = sg.kind == SIGN_REC_X ? s_recw[kk * rs + sg.rec] : ~0ull;
+                        const u64 m = sg.kind >= SIGN_REC_X ? s_recw[kk * rs + sg.rec] : ~0ull;
                         if (m) rd ^= m & prop_parity(seg, pbase + it, t);
                     } else {
                         const NoiseEntry e = ent[it - nsg];

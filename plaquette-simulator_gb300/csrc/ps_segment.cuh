@@ -40,9 +40,10 @@ struct SegGate {
 };
 
 // A sign operation r ^= (fx & z_a) ^ (fz & x_a): the Pauli gates (constant
-// masks, GateFunctors.hpp:303-307,323-327,372-376) and the X of a reset
-// (mask = record outcome).
-enum SignKind : int32_t { SIGN_X = 0, SIGN_Y = 1, SIGN_Z = 2, SIGN_REC_X = 3 };
+// masks, GateFunctors.hpp:303-307,323-327,372-376), the X of a reset and the
+// conditional X / Z that a program spells as H S S H / S S with a record as
+// flag (mask = record outcome).
+enum SignKind : int32_t { SIGN_X = 0, SIGN_Y = 1, SIGN_Z = 2, SIGN_REC_X = 3, SIGN_REC_Z = 4 };
 struct SegSign {
     uint16_t a;
     uint16_t kind;
@@ -117,7 +118,7 @@ struct SegmentDev {
     int32_t nq;
     int32_t ngates;
     int32_t nsigns;
-    // Reset-X sign ops carry a slot number (SegSign.rec); the record behind
+    // Record-flagged sign ops carry a slot number (SegSign.rec); the record behind
     // slot i is recsig_rec[i].  Their outcome words are staged per tile.
     const int32_t *recsig_rec;
     int32_t nrecsig;

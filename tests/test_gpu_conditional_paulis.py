@@ -1,0 +1,79 @@
+"""Conditional Paulis: programs undo an outcome with H S S H (X) or S S (Z)
+on one qubit with one record as flag, and the compiled forms apply those as
+sign flips.  Runs of conditional gates drawn so that such patterns appear
+whole, cut short, overlapping (S S S, H S S S H), split by another op on the
+qubit, with records changing midway and interleaved over qubits: records and
+tableau bit for bit against the oracle."""
+import numpy as np
+import pytest
+
+
+def conditional_circuit(n, seed, ops=160, flags_only_pauli=False):
+    from plaquette_simulator import circuits as C
+    rng = C.SplitMix64(seed)
+    c = C.Circuit(n)
+    for q in range(n):
+        c.h(q)
+    nrec = 0
+    for q in range(n):
+        c.m(q)
+        nrec += 1
+    todo = []  # conditional gates still to emit, per qubit, so that qubits interleave
+    for _ in range(ops):
+        k = rng.below(10)
+        a, b = rng.below(n), rng.below(n)
+        if k < 5:
+            rec = rng.below(nrec)
+            whole = (("H", "S", "S", "H"), ("S", "S"))
+            more = (("S",), ("H",), ("S", "S", "S"), ("H", "S", "S", "S", "H"), ("H", "S"), ("S", "H", "S", "S", "H"))
+            pat = whole[rng.below(2)] if flags_only_pauli or rng.below(2) else more[rng.below(len(more))]
+            todo += [(a, g, rec) for g in pat]
+            if flags_only_pauli or rng.below(3):  # emitted at once, or later among other qubits' gates
+                for q, g, r in todo:
+                    (c.h_if if g == "H" else c.s_if)(q, r)
+                todo = []
+        elif k == 5:
+            c.h(a)
+            c.pauli1(a, 0.05, 0.1, 0.02)
+        elif k == 6 and a != b:
+            c.cx(a, b)
+            c.pauli2(a, b, [0.01] * 15)
+        elif k == 7:
+            c.s(a)
+        elif k == 8:
+            (c.m if rng.below(2) else c.r)(a)
+            nrec += 1
+        else:
+            (c.x, c.y, c.z)[rng.below(3)](a)
+    for q, g, r in todo:
+        (c.h_if if g == "H" else c.s_if)(q, r)
+    for q in range(n):
+        c.m(q)
+    return c
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 3, 9, 33])
+@pytest.mark.parametrize("form", ["warp", "resident", "word_vector", "plain"])
+def test_conditional_paulis_match_oracle(ps, O, n, form):
+    from plaquette_simulator.circuit import CompiledCircuit
+    for seed in range(3):
+        c = conditional_circuit(n, 100 * n + seed)
+        shots = 64 * (1 + seed) + 13 * seed
+        st = ps.CliffordState(n, shots, 5 + seed, True)
+        cc = CompiledCircuit(c, st, fused=form != "plain", resident=form == "resident",
+                             word_vector=form == "word_vector")
+        o = O.Oracle(n, shots, seed=5 + seed)
+        nm = c.num_measurements()
+        for k in range(2):  # the second run goes on from the first one's tableau
+            cc.run()
+            table = c.op_array()
+            table[table[:, 0] >= 11, 3] += k * nm  # the oracle numbers its records over both runs
+            o.run(table, c.param_array())
+            gx, gz, gr = st.device_to_host_numpy()
+            ox, oz, orr = o.tableau()
+            assert np.array_equal(gx, ox) and np.array_equal(gz, oz) and np.array_equal(gr, orr)
+        for k in range(nm):
+            res, det = st.record(cc.first_record + k)
+            ores, odet = o.record(nm + k)
+            assert np.array_equal(res, ores) and np.array_equal(det, odet), k
