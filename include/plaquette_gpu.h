@@ -265,9 +265,11 @@ ps_status ps_circuit_destroy(ps_circuit *c);
 
 /* Per-kernel-kind device time of one run, measured with CUDA events around
  * every launch (the plan is enqueued launch by launch, not as a graph, and
- * the call waits for it).  Kinds: 0 tableau init, 1 channel sampling (fused),
- * 2 fused segment, 3 measurement, 4 per-op gate, 5 per-op channel, 6 sign
- * program (shared x/z), 7 x / z broadcast (shared x/z). */
+ * the call waits for it).  Kinds: 0 tableau init (in a run without reset: the
+ * pass that finds whether the shots share their x / z), 1 channel sampling
+ * (fused), 2 fused segment (and the walk of shared x / z through the circuit,
+ * where the host does not know them), 3 measurement, 4 per-op gate, 5 per-op
+ * channel, 6 sign program (shared x/z), 7 x / z broadcast (shared x/z). */
 #define PS_PROFILE_KINDS 8
 typedef struct {
     double ms[PS_PROFILE_KINDS];

@@ -21,6 +21,7 @@
 #include "ps_frame_dev.h"
 #include "ps_internal.h"
 #include "ps_segment.cuh"
+#include "ps_walk.h"
 
 namespace ps {
 
@@ -39,11 +40,12 @@ __global__ void detector_kernel(const u64 *__restrict__ res, int64_t w, const ui
     }
 }
 
-__global__ void set_params_kernel(RunParams *p, uint64_t seed, uint64_t event_base, uint64_t word_base) {
+__global__ void set_params_kernel(RunParams *p, uint64_t seed, uint64_t event_base, uint64_t word_base,
+                                  uint64_t valid) {
     p->seed = seed;
     p->event_base = event_base;
     p->word_base = word_base;
-    p->pad = 0;
+    p->valid = valid;
 }
 
 enum StepKind { K_GATE, K_CHANNEL, K_MEAS, K_SEGMENT, K_INIT };
@@ -207,6 +209,13 @@ struct ps_circuit {
     BroadcastJobDev fbjob{};
     cudaStream_t fstream = nullptr;  // the broadcast's side stream
     cudaEvent_t fev[2] = {nullptr, nullptr};
+    // The walk (ps_walk.h) of the runs it covers: those of circuits without
+    // per-shot conditional Cliffords, where the shared-x/z plan does not
+    // run.  Built with the per-shot plan's device tables.
+    bool own_tiles = false;          // the caller chose per-shot tiles: those kernels run
+    bool walk_ok = false;
+    WalkDev wdev{};
+    FrameTable wtable;               // its channel noise and x / z broadcast
     // ps_circuit_copy_records_async: the copy stream (own or the caller's),
     // the end of the run it copies, the end of the copy, and the error word
     // in pinned host memory.
@@ -881,13 +890,14 @@ struct Profiler {
 
 enum ProfKind { P_INIT = 0, P_SAMPLE = 1, P_SEGMENT = 2, P_MEASURE = 3, P_GATE = 4, P_CHANNEL = 5, P_FRAME = 6, P_BROADCAST = 7 };
 
-// Enqueues plan steps [from, to) on `st`.
 // The per-shot plan's device schedules and channel scratch: built on first
 // use -- a run without reset, measurement statistics, the tile tuner, or at
 // compile time when the shared-x/z plan does not apply -- so circuits that
 // only run from |0...0> in the shared-x/z plan never upload them.  Not
 // during stream capture (it uploads with synchronous copies).
 int build_segments_dev(ps_circuit *c);
+bool walk_covers(const ps_circuit *c);
+int build_walk(ps_circuit *c);
 int ensure_segments_dev(ps_circuit *c) {
     if (c->seg_dev_ready || c->opts.mode != PS_MODE_FUSED) return OK;
     if (c->h->signs_only) return fail(E_STATE, "a signs-only state runs only the shared-x/z plan");
@@ -895,6 +905,11 @@ int ensure_segments_dev(ps_circuit *c) {
         return fail(c->seg_dev_status, "the per-shot plan of this circuit does not fit its kernels");
     c->seg_dev_status = build_segments_dev(c);
     c->seg_dev_ready = c->seg_dev_status == OK;
+    if (c->seg_dev_ready && walk_covers(c)) {
+        const int rc = build_walk(c);
+        if (rc == E_CUDA) return c->seg_dev_status = rc;
+        if (rc != OK) set_error("");  // (no memory or tables for it: the per-shot kernels run)
+    }
     return c->seg_dev_status;
 }
 
@@ -968,7 +983,9 @@ int build_segments_dev(ps_circuit *c) {
     return OK;
 }
 
-int enqueue_steps(ps_circuit *c, cudaStream_t st, size_t from, size_t to, Profiler *prof = nullptr) {
+// Enqueues plan steps [from, to) on `st` (bad: launch_measure_list).
+int enqueue_steps(ps_circuit *c, cudaStream_t st, size_t from, size_t to, Profiler *prof = nullptr,
+                  const int32_t *bad = nullptr) {
     ps_state *h = c->h;
     auto timed = [&](int kind, auto &&launch) -> int {
         if (prof && prof->begin(kind) != OK) return E_CUDA;
@@ -996,16 +1013,16 @@ int enqueue_steps(ps_circuit *c, cudaStream_t st, size_t from, size_t to, Profil
             rc = timed(P_MEASURE, [&] {
                 return launch_measure_list(st, h->X, h->Z, h->R, h->n, h->w, c->d_meas + s.first, s.count,
                                            (uint64_t)h->seed, (uint64_t)h->word_base, c->d_params,
-                                           c->opts.meas_words);
+                                           c->opts.meas_words, bad);
             });
             break;
         case K_SEGMENT: {
             const SegHost &sg = c->segs[(size_t)s.first];
-            if (!sg.slots.empty()) rc = timed(P_SAMPLE, [&] { return launch_noise_sample(st, sg.dev, h->w, c->d_params); });
+            if (!sg.slots.empty()) rc = timed(P_SAMPLE, [&] { return launch_noise_sample(st, sg.dev, h->w, c->d_params, bad); });
             if (rc == OK)
                 rc = timed(P_SEGMENT, [&] {
                     return launch_segment(st, h->X, h->Z, h->R, h->n, h->w, sg.dev, c->opts.seg_rows,
-                                          c->opts.seg_words, c->opts.seg_threads, c->d_recs);
+                                          c->opts.seg_words, c->opts.seg_threads, c->d_recs, bad);
                 });
             break;
         }
@@ -1024,12 +1041,11 @@ int enqueue_steps(ps_circuit *c, cudaStream_t st, size_t from, size_t to, Profil
 // the sign kernel's shared memory; ranges that would need more read them
 // from global memory.  E_ARG: the program does not fit this kernel (the
 // per-shot plan runs instead).
-int frame_job_ranges(ps_circuit *c, FrameJobDev &job, std::vector<FrameRangeDev> &ranges,
+int frame_job_ranges(ps_circuit *c, const FrameProgram &P, FrameJobDev &job, std::vector<FrameRangeDev> &ranges,
                      std::vector<FrameSlotDev> &slots, std::vector<uint32_t> &s64, std::vector<uint32_t> &events,
                      std::vector<int32_t> &nv_range, std::vector<FrameChanTab> &ctabs,
                      std::vector<uint32_t> &surv) {
     ps_state *h = c->h;
-    const FrameProgram &P = c->fprog;
     ranges.clear();
     uint32_t max_rand = 0, max_scratch = 0, max_slots = 0;
     // channel records (indexed like slot_off) and the distinct tables
@@ -1161,6 +1177,263 @@ int frame_job_ranges(ps_circuit *c, FrameJobDev &job, std::vector<FrameRangeDev>
     return OK;
 }
 
+// Whether the walk runs a fused circuit's per-shot runs: no per-shot
+// conditional Clifford is left in its segments (flagged_paulis), the register
+// fits one CTA, and nobody asked for the per-shot kernels.  A pooled state's
+// bytes are bounded by its job's estimate, which does not count the walk's
+// tables.
+bool walk_covers(const ps_circuit *c) {
+    const ps_state *h = c->h;
+    if (c->opts.per_shot_xz || c->own_tiles || c->opts.seg_resident || h->pool) return false;
+    if (h->n < 1 || h->n > kWalkMaxQubits || walk_smem_bytes(h->n) > kSegSmemMax - 8192) return false;
+    size_t layers = 0;
+    for (const SegHost &sg : c->segs) {
+        layers += sg.layers.size();
+        for (const SegGate &g : sg.gates)
+            if ((g.code_rec & 15) == OP_H_IF || (g.code_rec & 15) == OP_S_IF) return false;
+    }
+    // The walk reads and writes the whole tableau once and costs a fraction
+    // of a microsecond a layer; the per-shot kernels pass over the touched
+    // columns segment by segment at about 2 TB/s, a launch each, and take a
+    // microsecond or more a measurement.  So short circuits on a few qubits
+    // of a large state stay with them.  Measured, per-shot kernels against
+    // walk: 3 rounds at d = 3, 64 shots 99 and 66 us; 9 rounds at d = 9, 64
+    // shots 1,123 and 230; 13 rounds at d = 13, 10,000 shots 13.7 and 0.74 ms;
+    // 90 distillation blocks, 16,384 shots 20.2 and 0.65 ms.
+    const double tableau = (double)h->W * (double)h->W * (double)h->w * 8.0, nm = (double)c->meas.size();
+    const double per_shot = 4.0 * (double)c->steps.size() + c->stats.segment_bytes / 2.0e6 + 1.0 * nm;
+    const double walk = 30.0 + 2.0 * tableau / 6.0e6 + 0.5 * (double)layers + 0.05 * nm;
+    return walk < per_shot;
+}
+
+// The walk's schedule from the per-shot plan's (the same layers on global
+// qubits, without the pad gates), the channel tables of its noise launch and
+// the arrays that the walk writes.
+int build_walk(ps_circuit *c) {
+    ps_state *h = c->h;
+    const int32_t n = (int32_t)h->n;
+    std::vector<WalkStep> steps;
+    std::vector<WalkPart> parts;
+    std::vector<uint32_t> gates, signs, slots;
+    std::vector<int32_t> mq(c->meas.size()), rec_of_op;
+    FrameProgram P;  // the launch ranges of the noise kernel, nothing else
+    int32_t nv = 0;
+    WalkPart part{-1, 0, 0, 0, 0};
+    auto close_part = [&] {
+        if (part.nv >= 0 || part.r1 > part.r0 || part.m1 > part.m0) parts.push_back(part);
+        part = WalkPart{-1, (int32_t)rec_of_op.size(), (int32_t)rec_of_op.size(), 0, 0};
+    };
+    for (const Step &s : c->steps) {
+        if (s.kind == K_SEGMENT) {
+            close_part();
+            const SegHost &sg = c->segs[(size_t)s.first];
+            const int nq = (int)sg.cols.size();
+            auto global = [&](int32_t l) { return (uint32_t)sg.cols[(size_t)l]; };
+            size_t sl = 0;
+            for (size_t l = 0; l < sg.layers.size(); ++l) {
+                const SegLayer &ly = sg.layers[l];
+                WalkStep w{};
+                w.i0 = (int32_t)gates.size();
+                for (int32_t r = ly.r0; r < ly.r1; ++r)
+                    for (int32_t g = sg.runs[(size_t)r].g0; g < sg.runs[(size_t)r].g1; ++g) {
+                        const SegGate &sgate = sg.gates[(size_t)g];
+                        if (sgate.a >= nq) continue;  // a pad lane
+                        const int32_t code = sgate.code_rec & 15;
+                        const bool two = code == OP_CX || code == OP_CZ;
+                        gates.push_back(walk_gate(global(sgate.a), two ? global(sgate.b) : 0u, (uint32_t)code));
+                    }
+                w.i1 = (int32_t)gates.size();
+                w.s0 = (int32_t)signs.size();
+                w.r0 = (int32_t)rec_of_op.size();
+                for (int32_t k = ly.s0; k < ly.s1; ++k) {
+                    const SegSign &sgn = sg.signs[(size_t)k];
+                    const uint32_t code = sgn.kind == SIGN_X       ? (uint32_t)OP_X
+                                          : sgn.kind == SIGN_Y     ? (uint32_t)OP_Y
+                                          : sgn.kind == SIGN_Z     ? (uint32_t)OP_Z
+                                          : sgn.kind == SIGN_REC_X ? kWalkRecX
+                                                                   : kWalkRecZ;
+                    uint32_t ord = 0;
+                    if (sgn.kind >= SIGN_REC_X) {
+                        ord = (uint32_t)rec_of_op.size() - (uint32_t)w.r0;
+                        if (ord >= kWalkMaxRecOps) return fail(E_ARG, "walk: too many record ops in a layer");
+                        rec_of_op.push_back(sg.recsig_rec[(size_t)sgn.rec]);
+                    }
+                    signs.push_back(walk_sign(global(sgn.a), code, ord));
+                }
+                w.s1 = (int32_t)signs.size();
+                w.n0 = (int32_t)slots.size();
+                for (; sl < sg.slots.size() && sg.slots[sl].layer == (int32_t)l; ++sl)
+                    slots.push_back(global(sg.slots[sl].a) |
+                                    (sg.slots[sl].b >= 0 ? global(sg.slots[sl].b) : 0xFFFFu) << 16);
+                w.n1 = (int32_t)slots.size();
+                if (w.i1 > w.i0 || w.s1 > w.s0 || w.n1 > w.n0) steps.push_back(w);
+            }
+            if (sl != sg.slots.size()) return fail(E_ARG, "walk: a channel outside its segment's layers");
+            part.r1 = (int32_t)rec_of_op.size();
+            if (!sg.slots.empty()) {
+                part.nv = nv++;
+                FrameProgram::Launch L{};
+                L.seg = s.first;
+                L.op0 = (uint32_t)P.ops.size();
+                L.op1 = L.op0 + 1;
+                FrameOp op{};
+                op.kind = F_NOISE;
+                op.arg = (int32_t)P.slot_off.size();
+                P.ops.push_back(op);
+                P.slot_off.resize(P.slot_off.size() + sg.slots.size() + 1, 0u);
+                P.launches.push_back(L);
+            }
+        } else if (s.kind == K_MEAS) {
+            WalkStep w{};
+            w.phase = 1;
+            w.i0 = s.first;
+            w.i1 = s.first + s.count;
+            steps.push_back(w);
+            std::set<int32_t> was_reset;
+            for (int32_t m = w.i0; m < w.i1; ++m) {
+                const int32_t q = c->meas[(size_t)m].q;
+                const bool again = was_reset.count(q) != 0;
+                if (again) was_reset.clear();  // a new run starts here
+                mq[(size_t)m] = q | (c->meas[(size_t)m].reset ? kWalkReset : 0) | (again ? kWalkBreak : 0);
+                if (c->meas[(size_t)m].reset) was_reset.insert(q);
+            }
+            part.m0 = w.i0;
+            part.m1 = w.i1;
+            close_part();
+        }
+    }
+    close_part();
+    WalkDev d{};
+    d.n = n;
+    d.ww = (int32_t)((h->W + 63) / 64);
+    d.nw = (int32_t)((h->n + 63) / 64);
+    d.nsteps = (int32_t)steps.size();
+    d.nparts = (int32_t)parts.size();
+    d.nm = (int32_t)c->meas.size();
+    d.w = h->w;
+    WalkStep *dst;
+    WalkPart *dp;
+    uint32_t *dg, *dsg, *dsl;
+    int32_t *dmq, *drec;
+    if (upload(h, c->owned, steps, &dst) || upload(h, c->owned, parts, &dp) || upload(h, c->owned, gates, &dg) ||
+        upload(h, c->owned, signs, &dsg) || upload(h, c->owned, slots, &dsl) || upload(h, c->owned, mq, &dmq) ||
+        upload(h, c->owned, rec_of_op, &drec))
+        return E_NOMEM;
+    d.steps = dst;
+    d.parts = dp;
+    d.gates = dg;
+    d.signs = dsg;
+    d.slots = dsl;
+    d.mq = dmq;
+    d.rec_of_op = drec;
+    d.meas = c->d_meas;
+    d.rp = c->d_params;
+    d.rec = c->d_res_block;
+    d.R = h->R;
+    // what the walk writes, one block
+    const size_t stride = (2 * (size_t)n + 1) & ~(size_t)1;  // even: read two rows at a time
+    const size_t ww = (size_t)d.ww, rows2 = (size_t)h->W * 2 * (size_t)d.nw;
+    const size_t words[] = {kWalkCtlBytes / sizeof(u64), rows2, rows2, slots.size() * 4 * ww, rec_of_op.size() * ww, c->meas.size(),
+                            c->meas.size() * 2 * ww, ww, (c->meas.size() * stride + 3) / 4};
+    size_t total = 0;
+    for (size_t v : words) total += v;
+    void *blk = nullptr;
+    if (dev_alloc(h, &blk, total * sizeof(u64)) != OK) return E_NOMEM;
+    c->owned.push_back(blk);
+    u64 *at = static_cast<u64 *>(blk);
+    PS_CUDA(cudaMemsetAsync(at, 0, (words[0] + words[1]) * sizeof(u64), h->stream));
+    auto take = [&](int i) {
+        u64 *p = at;
+        at += words[i];
+        return p;
+    };
+    u64 *const ctl = take(0);
+    d.bad = reinterpret_cast<int32_t *>(ctl);
+    d.gin = reinterpret_cast<uint64_t *>(take(1));
+    d.xz = reinterpret_cast<uint64_t *>(take(2));
+    d.smask = take(3);
+    d.rmask = take(4);
+    static_assert(sizeof(WalkMeas) == sizeof(u64), "one word a measurement");
+    d.minfo = reinterpret_cast<WalkMeas *>(take(5));
+    d.mmask = take(6);
+    d.fmask = take(7);
+    d.mlist = reinterpret_cast<uint16_t *>(take(8));
+    d.list_stride = (int64_t)stride;
+    FrameTable t;
+    t.masks = true;
+    t.off = d.bad;
+    t.njobs = 1;
+    t.bctr = reinterpret_cast<unsigned long long *>(ctl + 16);
+    if (nv > 0) {  // the channel noise of every segment and shot-word
+        FrameJobDev job{};
+        std::vector<FrameRangeDev> ranges;
+        std::vector<FrameSlotDev> fslots;
+        std::vector<uint32_t> fs64, fev, surv;
+        std::vector<int32_t> nvr;
+        std::vector<FrameChanTab> ctabs;
+        int rc = frame_job_ranges(c, P, job, ranges, fslots, fs64, fev, nvr, ctabs, surv);
+        if (rc != OK) return rc;
+        uint32_t ord = 0;  // the channel's place in smask
+        for (const FrameRangeDev &r : ranges)
+            for (int32_t q = 0; q < r.nslots; ++q) fslots[(size_t)r.rec_base + (size_t)q].t0 = ord++;
+        FrameRangeDev *dr;
+        FrameSlotDev *dfs;
+        uint32_t *ds64, *dev, *dsv;
+        FrameChanTab *dct;
+        int32_t *dnvr;
+        if (upload(h, c->owned, ranges, &dr) || upload(h, c->owned, fslots, &dfs) || upload(h, c->owned, fs64, &ds64) ||
+            upload(h, c->owned, fev, &dev) || upload(h, c->owned, ctabs, &dct) || upload(h, c->owned, surv, &dsv) ||
+            upload(h, c->owned, nvr, &dnvr))
+            return E_NOMEM;
+        job.ranges = dr;
+        job.slot = dfs;
+        job.slot_s64 = ds64;
+        job.slot_event = dev;
+        job.ctab = dct;
+        job.surv = dsv;
+        job.nv_range = dnvr;
+        job.smask = d.smask;
+        job.ww = d.ww;
+        job.nvec = c->fjob.nvec;  // (a run takes one plan or the other)
+        if (!job.nvec) {
+            void *pn = nullptr;
+            if (dev_alloc(h, &pn, (size_t)nv * (size_t)h->w * (size_t)frame_wp(h->n) * sizeof(u64)) != OK) return E_NOMEM;
+            c->owned.push_back(pn);
+            job.nvec = static_cast<u64 *>(pn);
+        }
+        d.nvec = job.nvec;
+        d.nvec_rows = frame_wp(h->n);
+        const std::vector<FrameJobDev> jobs{job};
+        const std::vector<int64_t> ncta0{0, (int64_t)nv * h->w};
+        FrameJobDev *dj;
+        int64_t *dn;
+        if (upload(h, c->owned, jobs, &dj) || upload(h, c->owned, ncta0, &dn)) return E_NOMEM;
+        t.jobs = dj;
+        t.ncta0 = dn;
+        t.nctas = ncta0[1];
+        t.nsmem = noise_job_smem(job);
+    }
+    const std::vector<BroadcastJobDev> bjobs{{h->X, h->Z, d.xz, h->n, h->w, (int64_t)d.nw}};
+    const std::vector<int64_t> chunk0{0, broadcast_chunks(h->n, h->w)};
+    BroadcastJobDev *db;
+    int64_t *dk;
+    if (upload(h, c->owned, bjobs, &db) || upload(h, c->owned, chunk0, &dk)) return E_NOMEM;
+    t.bjobs = db;
+    t.chunk0 = dk;
+    t.chunks = chunk0[1];
+    if (!c->fstream && cudaStreamCreateWithFlags(&c->fstream, cudaStreamNonBlocking) != cudaSuccess)
+        return cuda_fail(cudaGetLastError(), "cudaStreamCreate");
+    for (cudaEvent_t &e : c->fev)
+        if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+            return cuda_fail(cudaGetLastError(), "cudaEventCreate");
+    // (runs may be launched on other streams than the one that uploads)
+    PS_CUDA(cudaStreamSynchronize(h->stream));
+    c->wdev = d;
+    c->wtable = t;
+    c->walk_ok = true;
+    return OK;
+}
+
 // The shared-x/z plan of a run from |0...0>: the noise vectors of every range
 // and shot-word, then the whole sign program as one launch, with the
 // broadcast of the final x / z bits (host-known, so it needs nothing else)
@@ -1265,11 +1538,105 @@ int tune_frame_table(const FrameTable &t, cudaStream_t st, cudaStream_t side, cu
     return OK;
 }
 
+// The graph that a stream is being captured into, null when it is not.
+cudaGraph_t capturing_graph(cudaStream_t st) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    cudaGraph_t g = nullptr;
+    const cudaGraphNode_t *deps = nullptr;
+    const cudaGraphEdgeData *edges = nullptr;
+    size_t nd = 0;
+    if (cudaStreamGetCaptureInfo(st, &cs, &id, &g, &deps, &edges, &nd) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return cs == cudaStreamCaptureStatusActive ? g : nullptr;
+}
+
+// Adds what `enqueue` puts on its stream to the graph being captured from
+// st, as a part that runs when the condition was set.
+template <class F> int capture_conditional(cudaStream_t st, cudaGraphConditionalHandle cond, F &&enqueue) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    cudaGraph_t g = nullptr;
+    const cudaGraphNode_t *deps = nullptr;
+    const cudaGraphEdgeData *edges = nullptr;
+    size_t nd = 0;
+    PS_CUDA(cudaStreamGetCaptureInfo(st, &cs, &id, &g, &deps, &edges, &nd));
+    cudaGraphNodeParams p = {};
+    p.type = cudaGraphNodeTypeConditional;
+    p.conditional.handle = cond;
+    p.conditional.type = cudaGraphCondTypeIf;
+    p.conditional.size = 1;
+    cudaGraphNode_t node = nullptr;
+    PS_CUDA(cudaGraphAddNode(&node, g, deps, edges, nd, &p));
+    cudaStream_t bs = nullptr;
+    PS_CUDA(cudaStreamCreateWithFlags(&bs, cudaStreamNonBlocking));
+    cudaError_t e = cudaStreamBeginCaptureToGraph(bs, p.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                                  cudaStreamCaptureModeThreadLocal);
+    int rc = e == cudaSuccess ? enqueue(bs) : cuda_fail(e, "cudaStreamBeginCaptureToGraph");
+    if (e == cudaSuccess) {
+        cudaGraph_t body = nullptr;
+        e = cudaStreamEndCapture(bs, &body);
+        if (rc == OK && e != cudaSuccess) rc = cuda_fail(e, "cudaStreamEndCapture");
+    }
+    cudaStreamDestroy(bs);
+    if (rc != OK) return rc;
+    PS_CUDA(cudaStreamUpdateCaptureDependencies(st, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
+    return OK;
+}
+
+// The walk: gather (runs without reset), walk, then noise and signs with
+// the x / z broadcast beside them.
+int enqueue_walk(ps_circuit *c, cudaStream_t st, bool reset, Profiler *prof, cudaGraphConditionalHandle fall) {
+    auto timed = [&](int kind, auto &&launch) -> int {
+        if (prof && prof->begin(kind) != OK) return E_CUDA;
+        int rc = launch();
+        if (prof && rc == OK && prof->end() != OK) return E_CUDA;
+        return rc;
+    };
+    NvtxRange range("ps shared-x/z walk");
+    FrameTable t = c->wtable;
+    if (reset) t.off = nullptr;
+    int rc = OK;
+    if (!reset) rc = timed(P_INIT, [&] { return launch_walk_gather(st, c->h->X, c->h->Z, c->wdev); });
+    if (rc == OK) rc = timed(P_SEGMENT, [&] { return launch_walk(st, c->wdev, reset, fall); });
+    if (rc != OK) return rc;
+    const bool beside = !prof && c->fstream;
+    if (beside) {
+        PS_CUDA(cudaEventRecord(c->fev[0], st));
+        PS_CUDA(cudaStreamWaitEvent(c->fstream, c->fev[0], 0));
+        rc = launch_broadcast_jobs(c->fstream, t, c->opts.bcast_ctas);
+    }
+    if (rc == OK) rc = timed(P_SAMPLE, [&] { return launch_noise_vectors(st, t); });
+    if (rc == OK) rc = timed(P_FRAME, [&] { return launch_walk_signs(st, c->wdev, reset); });
+    if (rc != OK) return rc;
+    if (beside) {
+        PS_CUDA(cudaEventRecord(c->fev[1], c->fstream));
+        PS_CUDA(cudaStreamWaitEvent(st, c->fev[1], 0));
+        return OK;
+    }
+    return timed(P_BROADCAST, [&] { return launch_broadcast_jobs(st, t, c->opts.bcast_ctas); });
+}
+
 int enqueue_plan(ps_circuit *c, cudaStream_t st, bool reset, Profiler *prof = nullptr) {
     if (reset && c->frame_ok && !c->force_per_shot) return enqueue_frame(c, st, prof);
     {
         int rc = ensure_segments_dev(c);  // (captures call it before they begin)
         if (rc != OK) return rc;
+    }
+    if (c->walk_ok && !c->force_per_shot) {
+        if (reset) return enqueue_walk(c, st, reset, prof, 0);
+        // Where x / z turn out not to be shared, the per-shot kernels run: in
+        // a graph as a conditional part, else as launches that do nothing
+        // when the walk has run (52 of those cost 0.05 to 0.1 ms at 13 rounds).
+        cudaGraph_t g = capturing_graph(st);
+        cudaGraphConditionalHandle fall = 0;
+        if (g) PS_CUDA(cudaGraphConditionalHandleCreate(&fall, g, 0, cudaGraphCondAssignDefault));
+        const int rc = enqueue_walk(c, st, reset, prof, fall);
+        if (rc != OK) return rc;
+        if (g) return capture_conditional(st, fall, [&](cudaStream_t s) { return enqueue_steps(c, s, 0, c->steps.size()); });
+        return enqueue_steps(c, st, 0, c->steps.size(), prof, c->wdev.bad);
     }
     if (reset) {
         if (prof && prof->begin(P_INIT) != OK) return E_CUDA;
@@ -1344,7 +1711,7 @@ RunParams begin_run(ps_circuit *c, bool reset) {
     p.seed = (uint64_t)h->seed;
     p.event_base = h->events;
     p.word_base = (uint64_t)h->word_base;
-    p.pad = 0;
+    p.valid = h->valid ? 1u : 0u;
     h->events += c->num_events;
     if (reset) h->valid = true;
     return p;
@@ -1380,7 +1747,8 @@ int autotune_frame(ps_circuit *c, double *tune_ms) {
             return OK;
         }
     }
-    set_params_kernel<<<1, 1, 0, h->stream>>>(c->d_params, (uint64_t)h->seed, h->events, (uint64_t)h->word_base);
+    set_params_kernel<<<1, 1, 0, h->stream>>>(c->d_params, (uint64_t)h->seed, h->events, (uint64_t)h->word_base,
+                                             h->valid ? 1u : 0u);
     PS_CUDA(cudaGetLastError());
     int fw = 8, bc = 1;
     int rc = tune_frame_table(c->ftable, h->stream, c->fstream, c->fev[0], c->fev[1], &fw, &bc, nullptr);
@@ -1447,7 +1815,8 @@ int autotune(ps_circuit *c, double *tune_ms) {
         }
     }
     const cudaStream_t st = h->stream;
-    set_params_kernel<<<1, 1, 0, st>>>(c->d_params, (uint64_t)h->seed, h->events, (uint64_t)h->word_base);
+    set_params_kernel<<<1, 1, 0, st>>>(c->d_params, (uint64_t)h->seed, h->events, (uint64_t)h->word_base,
+                                             h->valid ? 1u : 0u);
     PS_CUDA(cudaGetLastError());
     auto prefix = [&](size_t upto) -> int {  // |0...0>, then steps [0, upto)
         int rc = launch_init_zero_on(st, h);
@@ -1555,6 +1924,7 @@ ps_status ps_circuit_compile(ps_state *h, const ps_op *ops_in, uint64_t nops, co
     auto *c = new ps_circuit;
     c->h = h;
     if (opts) c->opts = *opts;
+    c->own_tiles = c->opts.seg_rows > 0 || c->opts.seg_words > 0 || c->opts.seg_threads > 0 || c->opts.meas_words > 0;
     const bool fused = c->opts.mode == PS_MODE_FUSED;
     auto bail = [&](int rc) {
         const std::string msg = ps_last_error();
@@ -1820,7 +2190,7 @@ ps_status ps_circuit_compile(ps_state *h, const ps_op *ops_in, uint64_t nops, co
             std::vector<int32_t> nvr;
             std::vector<FrameChanTab> ctabs;
             std::vector<uint32_t> surv;
-            const int jrc = frame_job_ranges(c, job, ranges, fslots, fs64, fev, nvr, ctabs, surv);
+            const int jrc = frame_job_ranges(c, c->fprog, job, ranges, fslots, fs64, fev, nvr, ctabs, surv);
             if (jrc == E_ARG) {
                 set_error("");  // the program does not fit the one-launch kernel: the per-shot plan runs
                 ok = false;
@@ -1924,6 +2294,8 @@ ps_status ps_circuit_compile(ps_state *h, const ps_op *ops_in, uint64_t nops, co
         }
     }
     st.launches_per_run += 1;  // run-parameter update
+    if (c->walk_ok)  // runs from |0...0>: the parameters, walk, noise vectors, signs, broadcast
+        st.launches_per_run = 4 + (c->wtable.nctas > 0 ? 1 : 0);
     if (c->frame_ok) {  // runs from |0...0>: the parameters, the sign kernel, the broadcast
         st.shared_xz = 1;
         // parameters, noise vectors (when there are channels), signs, broadcast (unless signs only)
@@ -2006,7 +2378,7 @@ ps_status ps_circuit_run(ps_circuit *c, int reset_state) {
     NvtxRange range("ps circuit run");
     if (c->copy_pending) PS_CUDA(cudaStreamWaitEvent(h->stream, c->ev_copied, 0));  // it rewrites those records
     const RunParams p = begin_run(c, reset_state != 0);
-    set_params_kernel<<<1, 1, 0, h->stream>>>(c->d_params, p.seed, p.event_base, p.word_base);
+    set_params_kernel<<<1, 1, 0, h->stream>>>(c->d_params, p.seed, p.event_base, p.word_base, p.valid);
     PS_CUDA(cudaGetLastError());
     if (!reset_state && c->opts.use_graph && !c->exec[0] && c->frame_ok && !h->signs_only &&
         c->seg_dev_status < 0) {
@@ -2028,7 +2400,7 @@ ps_status ps_circuit_profile(ps_circuit *c, int reset_state, ps_circuit_profile_
     ps_state *h = c->h;
     std::memset(out, 0, sizeof(*out));
     const RunParams p = begin_run(c, reset_state != 0);
-    set_params_kernel<<<1, 1, 0, h->stream>>>(c->d_params, p.seed, p.event_base, p.word_base);
+    set_params_kernel<<<1, 1, 0, h->stream>>>(c->d_params, p.seed, p.event_base, p.word_base, p.valid);
     PS_CUDA(cudaGetLastError());
     Profiler prof;
     prof.st = h->stream;
@@ -2058,7 +2430,7 @@ ps_status ps_circuit_measure_stats(ps_circuit *c, int reset_state, int32_t *rand
     PS_CUDA(cudaStreamSynchronize(h->stream));
     PS_CUDA(cudaMemcpy(c->d_meas, m.data(), nm * sizeof(MeasOp), cudaMemcpyHostToDevice));
     const RunParams p = begin_run(c, reset_state != 0);
-    set_params_kernel<<<1, 1, 0, h->stream>>>(c->d_params, p.seed, p.event_base, p.word_base);
+    set_params_kernel<<<1, 1, 0, h->stream>>>(c->d_params, p.seed, p.event_base, p.word_base, p.valid);
     c->force_per_shot = true;  // the statistics come from the per-shot measurement kernel
     int rc = enqueue_plan(c, h->stream, reset_state != 0);
     c->force_per_shot = false;
@@ -2266,7 +2638,7 @@ RunParams circuit_current_params(const ps_circuit *c) {
     p.seed = (uint64_t)c->h->seed;
     p.event_base = c->h->events;
     p.word_base = (uint64_t)c->h->word_base;
-    p.pad = 0;
+    p.valid = c->h->valid ? 1u : 0u;
     return p;
 }
 RunParams circuit_begin_run(ps_circuit *c, bool reset) { return begin_run(c, reset); }

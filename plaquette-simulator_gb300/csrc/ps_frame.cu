@@ -57,29 +57,6 @@ __device__ __forceinline__ int job_of(const int64_t *__restrict__ first, int njo
     return lo;
 }
 
-// Bits 4 sub .. 4 sub + 3 of a random measurement's 64 outcomes of word k
-// (Philox block `sub`, or the forced bits) -- outcome_bits split over 16
-// lanes, so that one warp draws two measurements at once.
-__device__ __forceinline__ u64 outcome_quarter(const MeasOp &op, int sub, uint64_t seed, uint64_t event_base,
-                                               int64_t k, uint64_t word_base) {
-    u64 bits = 0ull;
-    if (op.forced) {
-        const u64 fw = op.forced[k];
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const int b = sub * 4 + l;
-            const float u = ((fw >> b) & 1ull) ? 0.25f : 0.75f;
-            if (u < op.bias) bits |= 1ull << b;
-        }
-    } else {
-        const u32x4 u = draw_block(seed, event_base + op.event, word_base + (uint64_t)k, (uint32_t)sub, TAG_MEASURE);
-#pragma unroll
-        for (int l = 0; l < 4; ++l)
-            if (unit_float(u.v[l]) < op.bias) bits |= 1ull << (sub * 4 + l);
-    }
-    return bits;
-}
-
 // One CTA of NW warps per (range with channels, shot-word) of a job: the
 // XOR its channel outcomes make on the signs of the word's 64 shots.  A
 // first pass draws every channel's first number (a Philox block gives the
@@ -90,11 +67,16 @@ __device__ __forceinline__ u64 outcome_quarter(const MeasOp &op, int sub, uint64
 // p = 1e-3) and lists the hit channels with their first numbers.  Then a
 // thread per hit samples its word (channel_word_est_hit: the same draws as
 // every other form) and flips its slot's rows in the sum (32-bit shared
-// atomics: XORs commute, and two slots may share a row).
-template <int NW>
+// atomics: XORs commute, and two slots may share a row).  MASKS: a slot's
+// rows are four bit masks over the rows (J.smask, written by the walk of
+// ps_walk.h) instead of a list; off: not 0 on the device when the launch has
+// nothing to do.
+template <int NW, bool MASKS>
 __global__ void __launch_bounds__(32 * NW) noise_vec_kernel(const FrameJobDev *__restrict__ jobs, int njobs,
-                                                            const int64_t *__restrict__ ncta0) {
+                                                            const int64_t *__restrict__ ncta0,
+                                                            const int32_t *__restrict__ off) {
     extern __shared__ __align__(16) u64 sm[];
+    if (MASKS && off && *off) return;
     constexpr int NT = 32 * NW;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int j = njobs > 1 ? job_of(ncta0, njobs, (int64_t)blockIdx.x) : 0;
@@ -204,9 +186,36 @@ __global__ void __launch_bounds__(32 * NW) noise_vec_kernel(const FrameJobDev *_
             shm[4 * l + 2] = m.fxb;
             shm[4 * l + 3] = m.fzb;
             sht0[l] = d.t0;
+            if (MASKS) len = (m.fxa | m.fza | m.fxb | m.fzb) != 0ull;
         }
         shlen[l] = len;
         __syncthreads();
+        if (MASKS) {
+            // (hit, word of the row masks) pairs over the threads; a mask is
+            // read only where the hit has that Pauli
+            const uint32_t ww = (uint32_t)J.ww;
+            for (uint32_t e = tid; e < (uint32_t)NT * ww; e += NT) {
+                const uint32_t lo = e / ww, t = e - lo * ww;
+                if (!shlen[lo]) continue;
+                const u64 fxa = shm[4 * lo + 0], fza = shm[4 * lo + 1], fxb = shm[4 * lo + 2], fzb = shm[4 * lo + 3];
+                const u64 *const mk = J.smask + (size_t)sht0[lo] * 4 * ww + t;
+                const u64 m0 = fxa ? mk[0] : 0ull, m1 = fza ? mk[ww] : 0ull;
+                const u64 m2 = fxb ? mk[2 * ww] : 0ull, m3 = fzb ? mk[3 * ww] : 0ull;
+                for (u64 v = m0 | m1 | m2 | m3; v; v &= v - 1) {
+                    const int b = __ffsll((long long)v) - 1;
+                    u64 f = 0ull;
+                    if ((m0 >> b) & 1ull) f ^= fxa;
+                    if ((m1 >> b) & 1ull) f ^= fza;
+                    if ((m2 >> b) & 1ull) f ^= fxb;
+                    if ((m3 >> b) & 1ull) f ^= fzb;
+                    unsigned *rw = reinterpret_cast<unsigned *>(&acc[64 * t + b]);
+                    if ((uint32_t)f) atomicXor(rw, (uint32_t)f);
+                    if (f >> 32) atomicXor(rw + 1, (uint32_t)(f >> 32));
+                }
+            }
+            __syncthreads();  // the chunk applied before the next one reuses its arrays
+            continue;
+        }
         // exclusive prefix of the row counts, in chunk order (thread tid
         // takes entry tid here)
         const uint32_t mine = shlen[tid];
@@ -522,7 +531,9 @@ __device__ __forceinline__ void broadcast_chunk(const BroadcastJobDev &B, int64_
 template <bool ONE>
 __global__ void __launch_bounds__(256, 8) broadcast_jobs_kernel(const BroadcastJobDev *__restrict__ jobs, int njobs,
                                                              const int64_t *__restrict__ chunk0, int64_t chunks,
-                                                             unsigned long long *ctr) {
+                                                             unsigned long long *ctr,
+                                                             const int32_t *__restrict__ off) {
+    if (off && *off) return;
     const int lane = threadIdx.x & 31;
     if (ctr) {
         for (;;) {
@@ -655,7 +666,8 @@ int launch_noise_vectors(cudaStream_t st, const FrameTable &t) {
     // CTAs (16K registers) find room beside them.
     const size_t smem = std::max<size_t>(t.nsmem, kNoiseSmemFloor);
     if (t.nctas > 0x7FFFFFFFll) return fail(E_ARG, "channel noise: too many (range, shot-word) pairs in one launch");
-    const void *kern = (const void *)noise_vec_kernel<kNoiseWarps>;
+    const void *kern = t.masks ? (const void *)noise_vec_kernel<kNoiseWarps, true>
+                               : (const void *)noise_vec_kernel<kNoiseWarps, false>;
     cudaLaunchConfig_t cfg;
     if (smem > 48 * 1024) {
         const int rc = allow_max_smem(kern);
@@ -674,7 +686,10 @@ int launch_noise_vectors(cudaStream_t st, const FrameTable &t) {
     attr[0].val.priority = g_prio_least;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    PS_CUDA(cudaLaunchKernelEx(&cfg, noise_vec_kernel<kNoiseWarps>, t.jobs, (int)t.njobs, t.ncta0));
+    if (t.masks)
+        PS_CUDA(cudaLaunchKernelEx(&cfg, noise_vec_kernel<kNoiseWarps, true>, t.jobs, (int)t.njobs, t.ncta0, t.off));
+    else
+        PS_CUDA(cudaLaunchKernelEx(&cfg, noise_vec_kernel<kNoiseWarps, false>, t.jobs, (int)t.njobs, t.ncta0, t.off));
     PS_CUDA(cudaGetLastError());
     return OK;
 }
@@ -721,9 +736,9 @@ int launch_broadcast_jobs(cudaStream_t st, const FrameTable &t, int ctas_per_sm)
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (t.njobs == 1)
-        PS_CUDA(cudaLaunchKernelEx(&cfg, broadcast_jobs_kernel<true>, t.bjobs, (int)t.njobs, t.chunk0, t.chunks, t.bctr));
+        PS_CUDA(cudaLaunchKernelEx(&cfg, broadcast_jobs_kernel<true>, t.bjobs, (int)t.njobs, t.chunk0, t.chunks, t.bctr, t.off));
     else
-        PS_CUDA(cudaLaunchKernelEx(&cfg, broadcast_jobs_kernel<false>, t.bjobs, (int)t.njobs, t.chunk0, t.chunks, t.bctr));
+        PS_CUDA(cudaLaunchKernelEx(&cfg, broadcast_jobs_kernel<false>, t.bjobs, (int)t.njobs, t.chunk0, t.chunks, t.bctr, t.off));
     PS_CUDA(cudaGetLastError());
     return OK;
 }

@@ -91,7 +91,10 @@ struct FrameJobDev {
     u64 *nvec;
     const int32_t *nv_range;
     int32_t nnv;
-    int32_t pad3;
+    // Row masks of the channels (ps_walk.h): channel slot t0 has masks
+    // smask[(4 t0 + c) * ww ..), c = rows with z(a), x(a), z(b), x(b).
+    int32_t ww;
+    const u64 *smask;
 };
 __host__ __device__ inline int64_t frame_wp(int64_t n) { return (2 * n + 2) & ~(int64_t)1; }
 
@@ -191,6 +194,8 @@ struct FrameTable {
     // two zeroed words (the broadcast's chunk counter and finished-CTA
     // count; zero again after every launch); null: a static chunk split
     unsigned long long *bctr = nullptr;
+    bool masks = false;            // the channels' rows are masks (FrameJobDev::smask)
+    const int32_t *off = nullptr;  // not 0 on the device: noise and broadcast launches do nothing
 };
 // Broadcast chunks a warp takes from the counter at a time.
 constexpr int64_t kBcastBatch = 8;

@@ -162,8 +162,11 @@ int check_channel_probs(const float *p, int count);
 struct RunParams;
 int launch_measure(ps_state *h, const MeasOp *ops_host, int nops);
 // words_per_cta: 1, 2 or 4 shot-words per CTA, 0 = automatic.
+// bad (here and below): a device word, null or not 0 for the launch to do
+// its work; 0 when another plan of the same run has done it (ps_walk.h).
 int launch_measure_list(cudaStream_t stream, u64 *X, u64 *Z, u64 *R, int64_t n, int64_t w, const MeasOp *dev_ops,
-                        int nops, uint64_t seed, uint64_t word_base, const RunParams *rp, int words_per_cta = 0);
+                        int nops, uint64_t seed, uint64_t word_base, const RunParams *rp, int words_per_cta = 0,
+                        const int32_t *bad = nullptr);
 
 // ps_segment.cu
 struct SegmentDev;
@@ -174,9 +177,9 @@ size_t segment_launch_smem(int nlayers, int nruns, int ngates, int nsigns, int n
 constexpr size_t kSegSmemMax = 227 * 1024;
 // slot_tags: entries carry their slot index instead of their layer.
 int launch_noise_sample(cudaStream_t stream, const SegmentDev &seg, int64_t w, const RunParams *rp,
-                        int slot_tags = 0);
+                        const int32_t *bad = nullptr, int slot_tags = 0);
 int launch_segment(cudaStream_t stream, u64 *X, u64 *Z, u64 *R, int64_t n, int64_t w, const SegmentDev &seg,
-                   int rows, int bw, int threads, const u64 *const *recs);
+                   int rows, int bw, int threads, const u64 *const *recs, const int32_t *bad = nullptr);
 
 // ps_frame.cu (shared-x/z runs; the launches are declared in ps_frame_dev.h)
 size_t frame_smem_bytes(int64_t n);

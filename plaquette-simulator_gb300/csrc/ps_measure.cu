@@ -759,8 +759,10 @@ __global__ void __launch_bounds__(NW * 32, 1) measure_kernel(u64 *X, u64 *Z, u64
                                                             const MeasOp *__restrict__ ops, int nops,
                                                             uint64_t seed_arg, uint64_t word_base_arg,
                                                             const RunParams *__restrict__ rp,
-                                                            int window_max, int use_cache) {
+                                                            int window_max, int use_cache,
+                                                            const int32_t *__restrict__ bad) {
     extern __shared__ u64 dyn[];
+    if (bad && !*bad) return;
     __shared__ Ctl ctl;
     const uint64_t seed = rp ? rp->seed : seed_arg;
     const uint64_t event_base = rp ? rp->event_base : 0ull;
@@ -927,7 +929,7 @@ size_t smem_bytes(int64_t n, int B, bool cache = false) {
 
 template <int B>
 int launch_b(cudaStream_t stream, u64 *X, u64 *Z, u64 *R, int64_t n, int64_t w, const MeasOp *dev_ops, int nops,
-             uint64_t seed, uint64_t word_base, const RunParams *rp, int window) {
+             uint64_t seed, uint64_t word_base, const RunParams *rp, int window, const int32_t *bad) {
     // The scan cache when the window path runs and it fits.
     const int cache = window > 0 && smem_bytes(n, B, true) <= kMeasSmemMax ? 1 : 0;
     const size_t smem = smem_bytes(n, B, cache != 0);
@@ -936,7 +938,7 @@ int launch_b(cudaStream_t stream, u64 *X, u64 *Z, u64 *R, int64_t n, int64_t w, 
         if (rc != OK) return rc;
     }
     measure_kernel<B><<<(unsigned)(w / B), NW * 32, smem, stream>>>(X, Z, R, n, w, dev_ops, nops, seed, word_base, rp,
-                                                                    window, cache);
+                                                                    window, cache, bad);
     PS_CUDA(cudaGetLastError());
     return OK;
 }
@@ -950,7 +952,8 @@ int measure_words_per_cta(int64_t n, int64_t w) {
 }
 
 int launch_measure_list(cudaStream_t stream, u64 *X, u64 *Z, u64 *R, int64_t n, int64_t w, const MeasOp *dev_ops,
-                        int nops, uint64_t seed, uint64_t word_base, const RunParams *rp, int words_per_cta) {
+                        int nops, uint64_t seed, uint64_t word_base, const RunParams *rp, int words_per_cta,
+                        const int32_t *bad) {
     if (nops <= 0) return OK;
     if (n > (int64_t)NW * 32 * MAXC) return fail(E_ARG, "too many qubits for the measurement kernel (max 2048)");
     // A single measurement has no window to overlap: spread it over the most
@@ -961,9 +964,9 @@ int launch_measure_list(cudaStream_t stream, u64 *X, u64 *Z, u64 *R, int64_t n, 
     if (nops > 1 && words_per_cta == 4 && w % 4 == 0 && smem_bytes(n, 4) <= kMeasSmemMax) B = 4;
     if (smem_bytes(n, B) > kMeasSmemMax) return fail(E_ARG, "measurement tile does not fit in shared memory");
     const int window = nops == 1 ? 0 : NW;
-    if (B == 4) return launch_b<4>(stream, X, Z, R, n, w, dev_ops, nops, seed, word_base, rp, window);
-    if (B == 2) return launch_b<2>(stream, X, Z, R, n, w, dev_ops, nops, seed, word_base, rp, window);
-    return launch_b<1>(stream, X, Z, R, n, w, dev_ops, nops, seed, word_base, rp, window);
+    if (B == 4) return launch_b<4>(stream, X, Z, R, n, w, dev_ops, nops, seed, word_base, rp, window, bad);
+    if (B == 2) return launch_b<2>(stream, X, Z, R, n, w, dev_ops, nops, seed, word_base, rp, window, bad);
+    return launch_b<1>(stream, X, Z, R, n, w, dev_ops, nops, seed, word_base, rp, window, bad);
 }
 
 int launch_measure(ps_state *h, const MeasOp *ops_host, int nops) {

@@ -24,7 +24,9 @@ namespace {
 
 // Pauli-channel sampling for one segment, pass 1: one thread per (word,
 // channel) draws the word's outcomes (channel_word) into dense[word][slot].
-__global__ void __launch_bounds__(256) noise_dense_kernel(SegmentDev seg, int64_t w, const RunParams *__restrict__ rp) {
+__global__ void __launch_bounds__(256) noise_dense_kernel(SegmentDev seg, int64_t w, const RunParams *__restrict__ rp,
+                                                         const int32_t *__restrict__ bad) {
+    if (bad && !*bad) return;
     const int64_t pair = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t k = pair / seg.nslots;
     const int s = (int)(pair - k * seg.nslots);
@@ -41,7 +43,9 @@ __global__ void __launch_bounds__(256) noise_dense_kernel(SegmentDev seg, int64_
 
 // Pass 2: one warp per word appends the non-identity outcomes to the word's
 // entry list; ballot compaction keeps slot (= layer) order.
-__global__ void __launch_bounds__(128) noise_compact_kernel(SegmentDev seg, int64_t w, int slot_tags) {
+__global__ void __launch_bounds__(128) noise_compact_kernel(SegmentDev seg, int64_t w, int slot_tags,
+                                                           const int32_t *__restrict__ bad) {
+    if (bad && !*bad) return;
     const int lane = threadIdx.x & 31;
     const int64_t k = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (k >= w) return;
@@ -324,8 +328,10 @@ template <int RC, int PB = 0>
 __global__ void __launch_bounds__(256, 2) segment_kernel(u64 *__restrict__ X, u64 *__restrict__ Z,
                                                         u64 *__restrict__ R, int64_t n, int64_t W, int64_t w,
                                                         SegmentDev seg, int rows, int bw, int64_t nchunks,
-                                                        int64_t ntiles, const u64 *const *__restrict__ recs) {
+                                                        int64_t ntiles, const u64 *const *__restrict__ recs,
+                                                        const int32_t *__restrict__ bad) {
     extern __shared__ u64 sm[];
+    if (bad && !*bad) return;
     const int nq = seg.nq;
     const int T = blockDim.x, tid = threadIdx.x;
     const int nq1 = seg_row_cells(nq);
@@ -707,13 +713,14 @@ size_t segment_launch_smem(int nlayers, int nruns, int ngates, int nsigns, int n
     return segment_smem_bytes(nq, rows, bw) + sched;
 }
 
-int launch_noise_sample(cudaStream_t stream, const SegmentDev &seg, int64_t w, const RunParams *rp, int slot_tags) {
+int launch_noise_sample(cudaStream_t stream, const SegmentDev &seg, int64_t w, const RunParams *rp, const int32_t *bad,
+                        int slot_tags) {
     if (seg.nslots == 0) return OK;
     const int64_t threads = (int64_t)seg.nslots * w;
-    noise_dense_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(seg, w, rp);
+    noise_dense_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(seg, w, rp, bad);
     PS_CUDA(cudaGetLastError());
     const int wpb = 4;
-    noise_compact_kernel<<<(unsigned)((w + wpb - 1) / wpb), 32 * wpb, 0, stream>>>(seg, w, slot_tags);
+    noise_compact_kernel<<<(unsigned)((w + wpb - 1) / wpb), 32 * wpb, 0, stream>>>(seg, w, slot_tags, bad);
     PS_CUDA(cudaGetLastError());
     return OK;
 }
@@ -721,7 +728,7 @@ int launch_noise_sample(cudaStream_t stream, const SegmentDev &seg, int64_t w, c
 namespace {
 template <int RC, int PB>
 int launch_segment_rc(cudaStream_t stream, u64 *X, u64 *Z, u64 *R, int64_t n, int64_t w, const SegmentDev &seg,
-                      int rows, int bw, int threads, const u64 *const *recs, size_t smem) {
+                      int rows, int bw, int threads, const u64 *const *recs, const int32_t *bad, size_t smem) {
     const int64_t W = 2 * n + 1;
     const int64_t nchunks = (w + bw - 1) / bw;
     const int64_t tiles = ((W + rows - 1) / rows) * nchunks;
@@ -739,14 +746,14 @@ int launch_segment_rc(cudaStream_t stream, u64 *X, u64 *Z, u64 *R, int64_t n, in
     if (per_sm < 1) return fail(E_ARG, "segment kernel does not fit on an SM");
     const int64_t grid = std::min<int64_t>(tiles, (int64_t)per_sm * g_num_sms);
     segment_kernel<RC, PB><<<(unsigned)grid, threads, smem, stream>>>(X, Z, R, n, W, w, seg, rows, bw, nchunks, tiles,
-                                                                   recs);
+                                                                   recs, bad);
     PS_CUDA(cudaGetLastError());
     return OK;
 }
 }  // namespace
 
 int launch_segment(cudaStream_t stream, u64 *X, u64 *Z, u64 *R, int64_t n, int64_t w, const SegmentDev &seg,
-                   int rows, int bw, int threads, const u64 *const *recs) {
+                   int rows, int bw, int threads, const u64 *const *recs, const int32_t *bad) {
     const bool wv = seg.word_vector && rows == 1 && seg.res_slots == 0;
     const size_t smem = segment_launch_smem(seg.nlayers, seg.nruns, wv ? 0 : seg.ngates, seg.nsigns, seg.nq,
                                             seg.nrecsig, rows, bw, seg.res_slots);
@@ -756,17 +763,17 @@ int launch_segment(cudaStream_t stream, u64 *X, u64 *Z, u64 *R, int64_t n, int64
     switch (seg.res_slots) {
     case 0:
         if (seg.word_vector && rows == 1) switch (bw) {  // the word-vector form
-            case 1: return launch_segment_rc<0, 1>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, smem);
-            case 2: return launch_segment_rc<0, 2>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, smem);
-            case 4: return launch_segment_rc<0, 4>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, smem);
-            case 8: return launch_segment_rc<0, 8>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, smem);
-            case 16: return launch_segment_rc<0, 16>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, smem);
+            case 1: return launch_segment_rc<0, 1>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, bad, smem);
+            case 2: return launch_segment_rc<0, 2>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, bad, smem);
+            case 4: return launch_segment_rc<0, 4>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, bad, smem);
+            case 8: return launch_segment_rc<0, 8>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, bad, smem);
+            case 16: return launch_segment_rc<0, 16>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, bad, smem);
             default: break;
             }
-        return launch_segment_rc<0, 0>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, smem);
-    case 2: return launch_segment_rc<2, 0>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, smem);
-    case 4: return launch_segment_rc<4, 0>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, smem);
-    case 8: return launch_segment_rc<8, 0>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, smem);
+        return launch_segment_rc<0, 0>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, bad, smem);
+    case 2: return launch_segment_rc<2, 0>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, bad, smem);
+    case 4: return launch_segment_rc<4, 0>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, bad, smem);
+    case 8: return launch_segment_rc<8, 0>(stream, X, Z, R, n, w, seg, rows, bw, threads, recs, bad, smem);
     default: return fail(E_ARG, "resident slots per lane must be 0, 2, 4 or 8");
     }
 }

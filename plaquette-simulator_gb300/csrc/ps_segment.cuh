@@ -10,7 +10,7 @@ struct RunParams {
     uint64_t seed;
     uint64_t event_base;
     uint64_t word_base;  // global index of the state's first 64-shot word
-    uint64_t pad;
+    uint64_t valid;      // 1: the tableau at the start is known to be a valid one (ps_state::valid)
 };
 
 // A tile row holds the nq columns of a segment and kSegDummyCols zero

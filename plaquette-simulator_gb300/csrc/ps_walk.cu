@@ -1,0 +1,731 @@
+// ps_walk.cu -- the kernels of ps_walk.h.
+#include <algorithm>
+
+#include "ps_draw.cuh"
+#include "ps_walk.h"
+
+namespace ps {
+
+namespace {
+
+constexpr unsigned kFull = 0xffffffffu;
+
+// Bits of word t that are rows [lo, hi).
+__device__ __forceinline__ u64 row_mask(int t, int lo, int hi) {
+    const int a = max(lo - 64 * t, 0), b = min(hi - 64 * t, 64);
+    if (a >= b) return 0ull;
+    const u64 m = b == 64 ? ~0ull : ((1ull << b) - 1ull);
+    return m & (~0ull << a);
+}
+
+__device__ __forceinline__ void smem_xor64(u64 *p, u64 v) {  // two 32-bit atomics (XOR has no carry)
+    unsigned *q = reinterpret_cast<unsigned *>(p);
+    if ((uint32_t)v) atomicXor(q, (uint32_t)v);
+    if (v >> 32) atomicXor(q + 1, (uint32_t)(v >> 32));
+}
+
+// A warp transposes 64 x 64 bits: lane l holds rows l (a) and l + 32 (b),
+// and ends with columns l and l + 32.
+__device__ __forceinline__ void transpose64(u64 &a, u64 &b, int lane) {
+    const u64 t = ((a >> 32) ^ b) & 0xFFFFFFFFull;
+    b ^= t;
+    a ^= t << 32;
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) {
+        const u64 m = s == 16  ? 0x0000FFFF0000FFFFull
+                      : s == 8 ? 0x00FF00FF00FF00FFull
+                      : s == 4 ? 0x0F0F0F0F0F0F0F0Full
+                      : s == 2 ? 0x3333333333333333ull
+                               : 0x5555555555555555ull;
+        const u64 oa = __shfl_xor_sync(kFull, a, s), ob = __shfl_xor_sync(kFull, b, s);
+        if (lane & s) {
+            a = (a & ~m) | ((oa >> s) & m);
+            b = (b & ~m) | ((ob >> s) & m);
+        } else {
+            a = (a & m) | ((oa & m) << s);
+            b = (b & m) | ((ob & m) << s);
+        }
+    }
+}
+
+// ------------------------------------------------------------- gather
+constexpr int kGatherUnroll = 4;  // 16-byte chunks of each plane in flight per thread
+
+// One bit of every (row, qubit), and whether all shots agree on it.  A row
+// of a plane is one stream of 16-byte chunks, `half` of them per qubit; a
+// CTA takes 1,024 consecutive chunks of a row, and a thread compares each
+// with its qubit's first word (in L1: its neighbours read it too), which
+// has to be all zeros or all ones.  The thread of a qubit's first chunk
+// notes the bit (out is zero before).  Bound by the one read of X and Z (d =
+// 15, 16,384 shots: 1.65 GB in 0.27 ms = 6.1 TB/s; a warp per 32 qubits with
+// lanes over each qubit's words: 0.38 ms); a mismatch stops the other CTAs at their next item.
+__global__ void __launch_bounds__(256) walk_gather_kernel(const u64 *__restrict__ X, const u64 *__restrict__ Z, int n,
+                                                         int W, int64_t w, uint32_t *__restrict__ out, int nw,
+                                                         int32_t *bad, const RunParams *__restrict__ rp) {
+    if (rp->valid == 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *bad = 1;
+        return;
+    }
+    const uint32_t half = (uint32_t)(w >> 1), chunks = (uint32_t)n * half;
+    const uint32_t per = 256u * kGatherUnroll, nblk = (chunks + per - 1) / per;
+    for (int64_t it = blockIdx.x; it < (int64_t)W * nblk; it += gridDim.x) {
+        if (*(volatile int32_t *)bad) return;
+        const uint32_t row = (uint32_t)(it / nblk), e0 = ((uint32_t)it - row * nblk) * per + threadIdx.x;
+        const u64 *const xr = X + (int64_t)row * n * w, *const zr = Z + (int64_t)row * n * w;
+        ulonglong2 vx[kGatherUnroll], vz[kGatherUnroll];
+        u64 hx[kGatherUnroll], hz[kGatherUnroll];
+        uint32_t q[kGatherUnroll];
+#pragma unroll
+        for (int u = 0; u < kGatherUnroll; ++u) {
+            const uint32_t e = min(e0 + 256u * u, chunks - 1);  // (past the end: the last chunk again)
+            q[u] = e / half;
+            vx[u] = *reinterpret_cast<const ulonglong2 *>(xr + 2ull * e);
+            vz[u] = *reinterpret_cast<const ulonglong2 *>(zr + 2ull * e);
+            hx[u] = xr[(int64_t)q[u] * w];
+            hz[u] = zr[(int64_t)q[u] * w];
+        }
+        bool fine = true;
+#pragma unroll
+        for (int u = 0; u < kGatherUnroll; ++u) {
+            fine &= vx[u].x == hx[u] && vx[u].y == hx[u] && vz[u].x == hz[u] && vz[u].y == hz[u];
+            fine &= hx[u] + 1ull <= 1ull && hz[u] + 1ull <= 1ull;  // all zeros or all ones
+            const uint32_t e = e0 + 256u * u;
+            if (e < chunks && e == q[u] * half) {
+                uint32_t *const o = out + (int64_t)row * 4 * nw + (q[u] >> 5);
+                if (hx[u]) atomicOr(o, 1u << (q[u] & 31u));
+                if (hz[u]) atomicOr(o + 2 * nw, 1u << (q[u] & 31u));
+            }
+        }
+        if (!fine) atomicOr(bad, 1);
+    }
+}
+
+// --------------------------------------------------------------- walk
+constexpr int kWalkThreads = 512;
+constexpr int kWalkWarps = kWalkThreads / 32;
+
+// Row strides in words: odd, so that the words of consecutive columns (or
+// rows) that a warp reads fall on distinct bank pairs.
+__host__ __device__ inline int walk_wp(int ww) { return ww | 1; }
+__host__ __device__ inline int walk_np(int nw) { return nw | 1; }
+
+struct WalkSmem {
+    size_t zc, f, stab, part, list, total;
+};
+__host__ __device__ inline WalkSmem walk_layout(int64_t n) {
+    const int ww = (int)((2 * n + 1 + 63) / 64), nw = (int)((n + 63) / 64);
+    const size_t col = (size_t)n * walk_wp(ww) * 8, st = 2 * (size_t)n * walk_np(nw) * 8;
+    WalkSmem L;
+    L.zc = col;
+    L.f = 2 * col;
+    L.stab = L.f + 16 * 8;
+    L.part = (L.stab + st + 15) & ~(size_t)15;
+    L.list = L.part + (size_t)kWalkWarps * 16 * 16;
+    L.total = L.list + (size_t)n * 4;
+    return L;
+}
+
+// One CTA follows one tableau through the circuit.  Its columns are bit
+// vectors over the rows, so a gate is a few words' XOR for all rows: half a
+// warp takes a gate, a lane per word, so that a column is one conflict-free
+// shared-memory access (lanes over gates instead measured 1.9x slower: 4-way
+// bank conflicts on the columns).  Nothing here scales with the shots: the
+// time is the warps' shared-memory accesses and instructions on one SM and
+// the latency of the steps (13 rounds at d = 13, 4,368 measurements: 0.33 ms,
+// about 1 us for a layer's gates, 1.2 us for its channels, 19 us for a phase
+// of 336 deterministic measurements; a random measurement on 450 qubits 1.4
+// us).
+//
+// A measurement phase goes position by position.  If its column has a
+// stabilizer row set, the measurement is random; every warp finds the pivot
+// by itself.  It multiplies the pivot row into every other row with x(q)
+// set, all rows of a word at once (bit-sliced mod-4 phase counters), over
+// the columns where the pivot row has a Pauli: two barriers.  Otherwise the
+// run of deterministic measurements from there on is done at once.  A
+// deterministic outcome is the product of the stabilizers that the column's
+// destabilizer rows select, its sign the summed phase of that product;
+// eight lanes take one measurement, a word of the row each, from a
+// row-major copy of the stabilizers that is made again after x / z changed.
+__global__ void __launch_bounds__(kWalkThreads, 1) walk_kernel(WalkDev d, int reset, cudaGraphConditionalHandle fall) {
+    extern __shared__ __align__(16) u64 sm[];
+    __shared__ int s_first[2], s_cnt[2];
+    __shared__ int32_t s_mq[kWalkThreads];
+    if (!reset && *d.bad) {  // the per-shot kernels' turn (a conditional part of the graph)
+        if (fall && threadIdx.x == 0) cudaGraphSetConditional(fall, 1u);
+        return;
+    }
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n = d.n, W = 2 * n + 1, ww = d.ww, nw = d.nw, wp = walk_wp(ww), np = walk_np(nw);
+    const WalkSmem SL = walk_layout(n);
+    char *const b8 = reinterpret_cast<char *>(sm);
+    u64 *const xc = sm, *const zc = reinterpret_cast<u64 *>(b8 + SL.zc);
+    u64 *const F = reinterpret_cast<u64 *>(b8 + SL.f);
+    u64 *const sx = reinterpret_cast<u64 *>(b8 + SL.stab), *const sz = sx + (size_t)n * np;
+    ulonglong2 *const part = reinterpret_cast<ulonglong2 *>(b8 + SL.part);  // a random one's phases: [warp][word]
+    uint32_t *const list = reinterpret_cast<uint32_t *>(b8 + SL.list);
+
+    for (int i = tid; i < n * wp; i += kWalkThreads) xc[i] = zc[i] = 0ull;
+    if (tid < 16) F[tid] = 0ull;
+    if (tid < 2) {
+        s_first[tid] = 0x7FFFFFFF;
+        s_cnt[tid] = 0;
+    }
+    __syncthreads();
+    if (reset) {  // |0...0>: x(i, i), z(i + n, i) and the scratch row's sign
+        for (int j = tid; j < n; j += kWalkThreads) {
+            xc[j * wp + (j >> 6)] = 1ull << (j & 63);
+            zc[j * wp + ((j + n) >> 6)] = 1ull << ((j + n) & 63);
+        }
+        if (tid == 0) F[(2 * n) >> 6] |= 1ull << ((2 * n) & 63);
+    } else {
+        for (int t = warp; t < ww * nw * 2; t += kWalkWarps) {
+            const int pl = t & 1, cb = (t >> 1) % nw, rb = (t >> 1) / nw;
+            const int r0 = rb * 64 + lane, r1 = r0 + 32;
+            u64 a = r0 < W ? d.gin[((int64_t)r0 * 2 + pl) * nw + cb] : 0ull;
+            u64 b = r1 < W ? d.gin[((int64_t)r1 * 2 + pl) * nw + cb] : 0ull;
+            transpose64(a, b, lane);
+            u64 *const c = pl ? zc : xc;
+            const int q0 = cb * 64 + lane, q1 = q0 + 32;
+            if (q0 < n) c[q0 * wp + rb] = a;
+            if (q1 < n) c[q1 * wp + rb] = b;
+        }
+    }
+    __syncthreads();
+
+    const u64 rm_stab = row_mask(lane, n, 2 * n), rm_destab = row_mask(lane, 0, n), rm_rows = row_mask(lane, 0, 2 * n);
+    // A step's ops as the threads hold them, fetched a step ahead (an op's
+    // load is several steps' work away): half-warp hw does ops hw, hw + HW,
+    // ..., and its lane t holds the one of round t.  Channels and sign ops
+    // past 16 rounds are read when due.
+    constexpr int HW = kWalkThreads / 16;
+    const int t = lane & 15, hw = tid >> 4;
+    const WalkStep none{};
+    auto step = [&](int i) { return i < d.nsteps ? d.steps[i] : none; };
+    auto held = [&](const uint32_t *ops, int o0, int o1) {
+        const int o = o0 + hw + HW * t;
+        return o < o1 ? ops[o] : 0u;
+    };
+    WalkStep st = step(0), st1 = step(1);
+    uint32_t hg = st.phase ? 0u : held(d.gates, st.i0, st.i1), hs = held(d.signs, st.s0, st.s1),
+             hn = held(d.slots, st.n0, st.n1);
+    bool dirty = true;  // the row-major stabilizers are stale
+    u64 fl = 0ull;      // the segment's constant flips, this thread's share of word t
+    int fi = 0, ci = 0;
+    for (int si = 0; si < d.nsteps; ++si) {
+        const WalkStep st2 = step(si + 2);
+        const uint32_t hg1 = st1.phase ? 0u : held(d.gates, st1.i0, st1.i1), hs1 = held(d.signs, st1.s0, st1.s1),
+                       hn1 = held(d.slots, st1.n0, st1.n1);
+        if (!st.phase) {
+            const int ng = st.i1 - st.i0;  // at most 511: disjoint qubits
+            for (int r = 0; r * HW < ng; ++r) {
+                const uint32_t o = __shfl_sync(kFull, hg, r, 16);
+                if (r * HW + hw >= ng || t >= ww) continue;
+                const uint32_t code = o >> 18;
+                const int ia = (int)(o & 511u) * wp + t, ib = (int)((o >> 9) & 511u) * wp + t;
+                const u64 x = xc[ia], z = zc[ia];
+                if (code >= OP_CX) {
+                    const u64 x2 = xc[ib], z2 = zc[ib];
+                    if (code == OP_CX) {
+                        fl ^= x & z2 & ~(x2 ^ z);
+                        xc[ib] = x2 ^ x;
+                        zc[ia] = z ^ z2;
+                    } else {
+                        fl ^= x & x2 & (z2 ^ z);
+                        zc[ib] = z2 ^ x;
+                        zc[ia] = z ^ x2;
+                    }
+                } else {
+                    fl ^= x & z;
+                    if (code == OP_H) xc[ia] = z;
+                    zc[ia] = code == OP_H ? x : z ^ x;
+                }
+            }
+            if (ng) __syncthreads();
+            // Pauli gates into the pending flips, record ops' rows out
+            for (int r = 0; st.s0 + r * HW < st.s1; ++r) {
+                const int g = st.s0 + r * HW + hw;
+                const uint32_t h = __shfl_sync(kFull, hs, r & 15, 16);
+                if (g >= st.s1 || t >= ww) continue;
+                const uint32_t o = r < 16 ? h : d.signs[g], code = (o >> 9) & 63u;
+                const int ia = (int)(o & 511u) * wp + t;
+                const u64 x = xc[ia], z = zc[ia];
+                if (code == OP_X) fl ^= z;
+                else if (code == OP_Y) fl ^= x ^ z;
+                else if (code == OP_Z) fl ^= x;
+                else d.rmask[(int64_t)(st.r0 + (int)(o >> 15)) * ww + t] = code == kWalkRecX ? z : x;
+            }
+            // channels: the rows that their Paulis flip
+            for (int r = 0; st.n0 + r * HW < st.n1; ++r) {
+                const int s = st.n0 + r * HW + hw;
+                const uint32_t h = __shfl_sync(kFull, hn, r & 15, 16);
+                if (s >= st.n1 || t >= ww) continue;
+                const uint32_t o = r < 16 ? h : d.slots[s], b = o >> 16;
+                const int ia = (int)(o & 0xFFFFu) * wp + t;
+                u64 *const out = d.smask + (int64_t)s * 4 * ww + t;
+                out[0] = zc[ia];
+                out[ww] = xc[ia];
+                if (b != 0xFFFFu) {
+                    out[2 * ww] = zc[(int)b * wp + t];
+                    out[3 * ww] = xc[(int)b * wp + t];
+                }
+            }
+            if (st.s1 > st.s0 || st.n1 > st.n0) __syncthreads();
+        }
+        if (st.phase) {  // the segment's constant flips, before a phase reads them
+            if (fl) smem_xor64(F + t, fl);
+            fl = 0ull;
+        } else {
+            dirty = true;
+        }
+        for (int c0 = st.i0; st.phase && c0 < st.i1; c0 += kWalkThreads) {
+            const int c1 = min(st.i1, c0 + kWalkThreads);
+            __syncthreads();
+            if (c0 + tid < c1) s_mq[tid] = d.mq[c0 + tid];
+            __syncthreads();
+            for (int pos = c0; pos < c1;) {
+                const int32_t mq = s_mq[pos - c0];
+                const int q = mq & kWalkQubit;
+                const u64 col = lane < ww ? xc[q * wp + lane] : 0ull;
+                const unsigned bal = __ballot_sync(kFull, (col & rm_stab) != 0ull);
+                if (bal) {
+                    // random: the lowest stabilizer row with x(q) set is the pivot
+                    const int src = __ffs(bal) - 1;
+                    const int p = 64 * src + __ffsll((long long)__shfl_sync(kFull, col & rm_stab, src)) - 1 - n;
+                    const int tp = p >> 6, tq = (p + n) >> 6;
+                    const u64 bp = 1ull << (p & 63), bq = 1ull << ((p + n) & 63);
+                    u64 Ml = col & rm_rows;
+                    if (lane == tp) Ml &= ~bp;
+                    if (lane == tq) Ml &= ~bq;
+                    const bool fp = (F[tq] & bq) != 0ull;
+                    const int j = tid;  // (n < 512)
+                    bool xp = false, zp = false;
+                    if (j < n) {
+                        xp = (xc[j * wp + tq] & bq) != 0ull;
+                        zp = (zc[j * wp + tq] & bq) != 0ull;
+                    }
+                    const unsigned lb = __ballot_sync(kFull, xp || zp);
+                    if (lb) {
+                        int base = 0;
+                        if (lane == 0) base = atomicAdd(&s_cnt[ci], __popc(lb));
+                        base = __shfl_sync(kFull, base, 0);
+                        if (xp || zp)
+                            list[base + __popc(lb & ((1u << lane) - 1u))] =
+                                (uint32_t)j | (xp ? 1u << 30 : 0u) | (zp ? 1u << 31 : 0u);
+                    }
+                    __syncthreads();
+                    // row p := the pivot row, row p + n := Z_q, the multiplied rows *= the pivot row
+                    if (j < n && !(xp || zp)) {
+                        xc[j * wp + tp] &= ~bp;
+                        zc[j * wp + tp] &= ~bp;
+                    }
+                    if (tid == 0) {
+                        s_cnt[ci ^ 1] = 0;
+                        F[tq] &= ~bq;
+                        F[tp] = (F[tp] & ~bp) | (fp ? bp : 0ull);
+                    }
+                    const int cnt = s_cnt[ci];
+                    const u64 M = __shfl_sync(kFull, Ml, t);
+                    u64 a1 = 0ull, a0 = 0ull;
+                    if (t < ww)
+                        for (int k = tid >> 4; k < cnt; k += kWalkThreads / 16) {
+                            const uint32_t v = list[k];
+                            const int jj = (int)(v & 0xFFFFu), o = jj * wp + t;
+                            const u64 x1 = xc[o], z1 = zc[o];
+                            const u64 x2 = v & (1u << 30) ? ~0ull : 0ull, z2 = v & (1u << 31) ? ~0ull : 0ull;
+                            phase_accumulate(x1, z1, x2, z2, M, a1, a0);
+                            u64 xn = x1 ^ (x2 & M), zn = z1 ^ (z2 & M);
+                            if (t == tp) {
+                                xn = (xn & ~bp) | (x2 & bp);
+                                zn = (zn & ~bp) | (z2 & bp);
+                            }
+                            if (t == tq) {
+                                xn &= ~bq;
+                                zn = (zn & ~bq) | (jj == q ? bq : 0ull);
+                            }
+                            xc[o] = xn;
+                            zc[o] = zn;
+                        }
+                    {
+                        const u64 e1 = __shfl_xor_sync(kFull, a1, 16), e0 = __shfl_xor_sync(kFull, a0, 16);
+                        phase_add(a1, a0, e1, e0);
+                    }
+                    if (lane < 16) part[warp * 16 + t] = make_ulonglong2(a1, a0);
+                    __syncthreads();
+                    if (warp < ww) {  // warp = word: the warps' partial counters (beside the next position's reads)
+                        const ulonglong2 v = part[(lane & (kWalkWarps - 1)) * 16 + warp];
+                        u64 b1 = v.x, b0 = v.y;
+#pragma unroll
+                        for (int o = kWalkWarps / 2; o > 0; o >>= 1) {
+                            const u64 e1 = __shfl_xor_sync(kFull, b1, o), e0 = __shfl_xor_sync(kFull, b0, o);
+                            phase_add(b1, b0, e1, e0);
+                        }
+                        b1 = __shfl_sync(kFull, b1, 0) ^ (fp ? ~0ull : 0ull);
+                        // this word's multiplied rows and constants into the list
+                        const u64 Mw = __shfl_sync(kFull, Ml, warp);
+                        const int before = __reduce_add_sync(kFull, lane < warp ? __popcll(Ml) : 0);
+                        uint16_t *const o = d.mlist + (int64_t)pos * d.list_stride + before;
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int bit = lane + 32 * h;
+                            if ((Mw >> bit) & 1ull)
+                                o[__popcll(Mw & ((1ull << bit) - 1ull))] =
+                                    (uint16_t)((64 * warp + bit) | (((b1 >> bit) & 1ull) ? 0x8000 : 0));
+                        }
+                        if (lane == 0 && (mq & kWalkReset))
+                            d.mmask[((int64_t)pos * 2 + 1) * ww + warp] = zc[q * wp + warp];
+                        const int rows = __reduce_add_sync(kFull, __popcll(Ml));
+                        if (tid == 0)
+                            d.minfo[pos] = WalkMeas{1u | (mq & kWalkReset ? 4u : 0u) | (uint32_t)p << 8, rows};
+                    }
+                    dirty = true;
+                    ci ^= 1;
+                    ++pos;
+                    continue;
+                }
+                // deterministic up to e: the next random measurement, or a qubit
+                // that the run has reset
+                {
+                    const int m = pos + 1 + tid;
+                    unsigned cand = 0x7FFFFFFFu;
+                    if (m < c1) {
+                        const int32_t v = s_mq[m - c0];
+                        const u64 *const c = xc + (v & kWalkQubit) * wp;
+                        u64 any = 0ull;
+                        for (int t = n >> 6; t < ww; ++t) any |= c[t] & row_mask(t, n, 2 * n);
+                        if (any || (v & kWalkBreak)) cand = (unsigned)m;
+                    }
+                    cand = __reduce_min_sync(kFull, cand);
+                    if (lane == 0 && cand != 0x7FFFFFFFu) atomicMin(&s_first[fi], (int)cand);
+                }
+                if (dirty) {  // stabilizer rows n .. 2n - 1, row-major
+                    const int rb0 = n >> 6, nrb = (2 * n + 63) / 64 - rb0;
+                    for (int t = warp; t < nrb * nw * 2; t += kWalkWarps) {
+                        const int pl = t & 1, cb = (t >> 1) % nw, rb = rb0 + (t >> 1) / nw;
+                        const u64 *const c = pl ? zc : xc;
+                        const int q0 = cb * 64 + lane, q1 = q0 + 32;
+                        u64 a = q0 < n ? c[q0 * wp + rb] : 0ull, b = q1 < n ? c[q1 * wp + rb] : 0ull;
+                        transpose64(a, b, lane);
+                        u64 *const o = pl ? sz : sx;
+                        const int i0 = rb * 64 + lane - n, i1 = i0 + 32;
+                        if (i0 >= 0 && i0 < n) o[i0 * np + cb] = a;
+                        if (i1 >= 0 && i1 < n) o[i1 * np + cb] = b;
+                    }
+                    dirty = false;
+                }
+                __syncthreads();
+                const int e = min(s_first[fi], c1);
+                fi ^= 1;
+                if (tid == 0) s_first[fi] = 0x7FFFFFFF;  // (every thread is past its last read)
+                const int gl = lane & 7;
+                const unsigned gmask = 0xFFu << (lane & 24);
+                const u64 rmd = __shfl_sync(kFull, rm_destab, gl);
+                for (int m = pos + (tid >> 3); m < e; m += kWalkThreads / 8) {
+                    const int32_t v = s_mq[m - c0];
+                    const int qm = v & kWalkQubit;
+                    const u64 mine = gl < nw ? xc[qm * wp + gl] & rmd : 0ull;  // destabilizer rows, 64 a lane
+                    if (gl < nw) d.mmask[(int64_t)m * 2 * ww + gl] = mine;
+                    int sum = 0;
+                    u64 ax = 0ull, az = 0ull;
+                    uint32_t c = 0;
+                    for (unsigned has = (__ballot_sync(gmask, mine != 0ull) >> (lane & 24)) & 0xFFu; has; has &= has - 1) {
+                        const int t = __ffs(has) - 1;
+                        for (u64 word = __shfl_sync(gmask, mine, t, 8); word; word &= word - 1) {
+                            const int i = 64 * t + __ffsll((long long)word) - 1;
+                            const u64 x = gl < nw ? sx[i * np + gl] : 0ull, z = gl < nw ? sz[i * np + gl] : 0ull;
+                            const u64 plus = (ax & ~az & x & z) | (ax & az & ~x & z) | (~ax & az & x & ~z);
+                            const u64 minus = (ax & az & x & ~z) | (ax & ~az & ~x & z) | (~ax & az & x & z);
+                            sum += __popcll(plus) - __popcll(minus);
+                            ax ^= x;
+                            az ^= z;
+                            c ^= (uint32_t)(F[(i + n) >> 6] >> ((i + n) & 63)) & 1u;
+                        }
+                    }
+                    __syncwarp(gmask);
+#pragma unroll
+                    for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(gmask, sum, o);
+                    c ^= ((uint32_t)sum >> 1) & 1u;
+                    if (v & kWalkReset)
+                        for (int t = gl; t < ww; t += 8)
+                            d.mmask[((int64_t)m * 2 + 1) * ww + t] = zc[qm * wp + t] & row_mask(t, 0, 2 * n);
+                    if (gl == 0) d.minfo[m] = WalkMeas{c << 1 | (v & kWalkReset ? 4u : 0u), e};
+                }
+                __syncthreads();
+                // the scratch row is the last one's product, Z on its qubit
+                const int ql = s_mq[e - 1 - c0] & kWalkQubit;
+                const int ts = (2 * n) >> 6;
+                const u64 bs = 1ull << ((2 * n) & 63);
+                if (tid < n) {
+                    xc[tid * wp + ts] &= ~bs;
+                    zc[tid * wp + ts] = (zc[tid * wp + ts] & ~bs) | (tid == ql ? bs : 0ull);
+                }
+                if (tid == 0) F[ts] &= ~bs;
+                pos = e;
+                // (the next reads of these words leave the scratch row out, and
+                // a barrier comes before their next write)
+            }
+        }
+        if (st.phase) __syncthreads();
+        st = st1;
+        st1 = st2;
+        hg = hg1;
+        hs = hs1;
+        hn = hn1;
+    }
+    if (fl) smem_xor64(F + t, fl);
+    __syncthreads();
+    // pending flips and final bits
+    if (tid < ww) d.fmask[tid] = F[tid];
+    for (int t = warp; t < ww * nw * 2; t += kWalkWarps) {
+        const int pl = t & 1, cb = (t >> 1) % nw, rb = (t >> 1) / nw;
+        const u64 *const c = pl ? zc : xc;
+        const int q0 = cb * 64 + lane, q1 = q0 + 32;
+        u64 a = q0 < n ? c[q0 * wp + rb] : 0ull, b = q1 < n ? c[q1 * wp + rb] : 0ull;
+        transpose64(a, b, lane);
+        const int r0 = rb * 64 + lane, r1 = r0 + 32;
+        if (r0 < W) d.xz[((int64_t)r0 * 2 + pl) * nw + cb] = a;
+        if (r1 < W) d.xz[((int64_t)r1 * 2 + pl) * nw + cb] = b;
+    }
+}
+
+// -------------------------------------------------------------- signs
+constexpr int kSignThreads = 512;
+constexpr int kSignChunk = 512;  // measurements whose info and outcomes are held at a time
+constexpr int kSignLists = 128;  // random measurements whose row lists are fetched at a time
+constexpr int kSignShort = 32;   // rows of a short list: one warp's lanes
+constexpr int kSignRows = 2;     // tableau rows per thread: 2 * 511 + 1 over 512 threads
+
+// One CTA per shot-word: its W signs stay in shared memory for the whole
+// run, as R XOR the constant flips that the walk carries.  The masks are the
+// same for every CTA (they stay in L2), so the time is the chain of steps: a
+// noise vector (fetched a segment ahead), the record ops, then runs of
+// deterministic measurements (eight lanes each, six in flight) and of random
+// ones (a chain: each reads rows that the ones before wrote).  13 rounds at
+// d = 13, 10,000 shots: 0.12 ms; 90 distillation blocks at 16,384 shots (630
+// random measurements): 0.21 ms, where a barrier and all rows a measurement
+// took 0.41.
+__global__ void __launch_bounds__(kSignThreads, 2) walk_signs_kernel(WalkDev d, int reset) {
+    extern __shared__ __align__(16) u64 sR[];  // [2n + 1]
+    __shared__ u64 sout[kSignChunk];           // drawn outcomes, then outcomes of deterministic measurements
+    __shared__ WalkMeas sinfo[kSignChunk];
+    __shared__ __align__(4) uint16_t slist[kSignLists * kSignShort];
+    __shared__ int snext;
+    if (!reset && *d.bad) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n = d.n, W = 2 * n + 1, ww = d.ww, nw = d.nw;
+    const int64_t w = d.w, k = blockIdx.x;
+    const RunParams rp = *d.rp;
+    for (int i = tid; i < W; i += kSignThreads) sR[i] = reset ? 0ull : d.R[(int64_t)i * w + k];
+    u64 nv[kSignRows];  // the next part's noise
+    auto fetch_nv = [&](int p) {
+        const int v = p < d.nparts ? d.parts[p].nv : -1;
+#pragma unroll
+        for (int u = 0; u < kSignRows; ++u) {
+            const int i = tid + u * kSignThreads;
+            nv[u] = v >= 0 && i < W ? d.nvec[((int64_t)v * w + k) * d.nvec_rows + i] : 0ull;
+        }
+    };
+    fetch_nv(0);
+    __syncthreads();
+    for (int pi = 0; pi < d.nparts; ++pi) {
+        const WalkPart P = d.parts[pi];
+#pragma unroll
+        for (int u = 0; u < kSignRows; ++u) {
+            const int i = tid + u * kSignThreads;
+            if (i < W) sR[i] ^= nv[u];
+        }
+        fetch_nv(pi + 1);
+        if (P.r1 > P.r0) {  // record ops: half a warp each, a lane per word
+            __syncthreads();
+            const int t = lane & 15;
+            constexpr int U = 6, step = kSignThreads / 16;
+            for (int r0 = P.r0 + (tid >> 4); r0 < P.r1; r0 += U * step) {
+                u64 m[U], f[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int r = r0 + u * step;
+                    const bool on = r < P.r1 && t < ww;
+                    m[u] = on ? d.rmask[(int64_t)r * ww + t] : 0ull;
+                    f[u] = on ? d.rec[(int64_t)d.rec_of_op[r] * w + k] : 0ull;
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (f[u])
+                        for (u64 v = m[u]; v; v &= v - 1) smem_xor64(sR + 64 * t + __ffsll((long long)v) - 1, f[u]);
+            }
+        }
+        for (int c0 = P.m0; c0 < P.m1; c0 += kSignChunk) {
+            const int c1 = min(P.m1, c0 + kSignChunk);
+            if (c0 > P.m0) __syncthreads();
+            if (c0 + tid < c1) sinfo[tid] = d.minfo[c0 + tid];
+            __syncthreads();
+            for (int m0 = c0 + 2 * warp; m0 < c1; m0 += 2 * (kSignThreads / 32)) {  // draws, two per warp
+                const int m = m0 + (lane >> 4), sub = lane & 15;
+                const bool on = m < c1 && (sinfo[m - c0].info & 1u);
+                if (!__any_sync(kFull, on)) continue;
+                u64 bits = 0ull;
+                if (on) bits = outcome_quarter(d.meas[m], sub, rp.seed, rp.event_base, k, rp.word_base);
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) bits |= __shfl_xor_sync(kFull, bits, o);
+                if (on && sub == 0) sout[m - c0] = bits;
+            }
+            __syncthreads();
+            for (int pos = c0; pos < c1;) {
+                const WalkMeas I = sinfo[pos - c0];
+                if (!(I.info & 1u)) {
+                    const int e = min(I.end, c1);
+                    const int gl = lane & 7;
+                    const unsigned gmask = 0xFFu << (lane & 24);
+                    constexpr int U = 6, step = kSignThreads / 8;
+                    for (int m0 = pos + (tid >> 3); m0 < e; m0 += U * step) {
+                        u64 word[U];
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            const int m = m0 + u * step;
+                            word[u] = m < e && gl < nw ? d.mmask[(int64_t)m * 2 * ww + gl] : 0ull;
+                        }
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            const int m = m0 + u * step;
+                            if (m >= e) break;
+                            u64 acc = 0ull;
+                            for (u64 v = word[u]; v; v &= v - 1) acc ^= sR[n + 64 * gl + __ffsll((long long)v) - 1];
+                            __syncwarp(gmask);
+#pragma unroll
+                            for (int o = 4; o > 0; o >>= 1) acc ^= __shfl_xor_sync(gmask, acc, o);
+                            if (gl == 0) {
+                                if (sinfo[m - c0].info & 2u) acc = ~acc;
+                                sout[m - c0] = acc;
+                                d.rec[(int64_t)m * w + k] = acc;
+                                d.rec[(int64_t)(d.nm + m) * w + k] = ~0ull;
+                            }
+                        }
+                    }
+                    __syncthreads();
+                    {  // the resets' X, after every read
+                        const int t = lane & 15;
+                        for (int m = pos + (tid >> 4); m < e; m += kSignThreads / 16) {
+                            if (!(sinfo[m - c0].info & 4u)) continue;
+                            const u64 f = sout[m - c0];
+                            if (f && t < ww)
+                                for (u64 v = d.mmask[((int64_t)m * 2 + 1) * ww + t]; v; v &= v - 1)
+                                    smem_xor64(sR + 64 * t + __ffsll((long long)v) - 1, f);
+                        }
+                    }
+                    // the scratch row: the last outcome, which its own reset clears
+                    if (tid == 0) sR[2 * n] = (sinfo[e - 1 - c0].info & 4u) ? 0ull : sout[e - 1 - c0];
+                    __syncthreads();
+                    pos = e;
+                    continue;
+                }
+                // random: R[p] := R[p+n], R[p+n] := outcome, R[i] ^= R[p] ^ c_i.
+                // Short row lists are warp 0's, one after the other (no
+                // barrier between them); the lists of a stretch of
+                // measurements come to shared memory first.
+                const int end = min(c1, pos + kSignLists);
+                for (int m = pos + (tid >> 4); m < end; m += kSignThreads / 16) {
+                    const int l = 2 * (lane & 15);
+                    const bool on = (sinfo[m - c0].info & 1u) && l < sinfo[m - c0].end;
+                    reinterpret_cast<uint32_t *>(slist)[(m - pos) * (kSignShort / 2) + (lane & 15)] =
+                        on ? *reinterpret_cast<const uint32_t *>(d.mlist + (int64_t)m * d.list_stride + l) : 0u;
+                }
+                __syncthreads();
+                if (warp == 0) {
+                    int m = pos;
+                    for (; m < end; ++m) {
+                        const WalkMeas J = sinfo[m - c0];
+                        if (!(J.info & 1u) || J.end > kSignShort) break;
+                        const int p = (int)(J.info >> 8);
+                        const uint32_t v = slist[(m - pos) * kSignShort + lane];
+                        const u64 rpv = sR[p + n], out = sout[m - c0];
+                        __syncwarp();
+                        if (lane < J.end) sR[v & 0x7FFFu] ^= rpv ^ ((v >> 15) ? ~0ull : 0ull);
+                        if (lane == 0) {  // (the list holds neither p nor p + n)
+                            sR[p] = rpv;
+                            sR[p + n] = out;
+                            d.rec[(int64_t)m * w + k] = out;
+                            d.rec[(int64_t)(d.nm + m) * w + k] = 0ull;
+                        }
+                        __syncwarp();
+                        if (J.info & 4u) {  // the reset's X
+                            if (lane < ww)
+                                for (u64 x = d.mmask[((int64_t)m * 2 + 1) * ww + lane]; x; x &= x - 1)
+                                    sR[64 * lane + __ffsll((long long)x) - 1] ^= out;
+                            __syncwarp();
+                        }
+                    }
+                    if (lane == 0) snext = m;
+                }
+                __syncthreads();
+                const int at = snext;
+                if (at < end && (sinfo[at - c0].info & 1u)) {  // a long list: every thread
+                    const WalkMeas J = sinfo[at - c0];
+                    const int p = (int)(J.info >> 8);
+                    const u64 rpv = sR[p + n], out = sout[at - c0];
+                    __syncthreads();
+                    for (int e = tid; e < J.end; e += kSignThreads) {
+                        const uint32_t v = d.mlist[(int64_t)at * d.list_stride + e];
+                        sR[v & 0x7FFFu] ^= rpv ^ ((v >> 15) ? ~0ull : 0ull);
+                    }
+                    if (tid == 0) {
+                        sR[p] = rpv;
+                        sR[p + n] = out;
+                        d.rec[(int64_t)at * w + k] = out;
+                        d.rec[(int64_t)(d.nm + at) * w + k] = 0ull;
+                    }
+                    __syncthreads();
+                    if (J.info & 4u) {
+                        const u64 *const zm = d.mmask + ((int64_t)at * 2 + 1) * ww;
+                        for (int i = tid; i < W; i += kSignThreads)
+                            if ((zm[i >> 6] >> (i & 63)) & 1ull) sR[i] ^= out;
+                        __syncthreads();
+                    }
+                    pos = at + 1;
+                } else {
+                    pos = at;
+                }
+            }
+        }
+        __syncthreads();
+    }
+    for (int i = tid; i < W; i += kSignThreads)
+        d.R[(int64_t)i * w + k] = sR[i] ^ (((d.fmask[i >> 6] >> (i & 63)) & 1ull) ? ~0ull : 0ull);
+}
+
+int g_walk_sms = 0;
+
+}  // namespace
+
+size_t walk_smem_bytes(int64_t n) { return walk_layout(n).total; }
+
+int launch_walk_gather(cudaStream_t st, const u64 *X, const u64 *Z, const WalkDev &d) {
+    if (g_walk_sms == 0) {
+        int dev = 0;
+        PS_CUDA(cudaGetDevice(&dev));
+        PS_CUDA(cudaDeviceGetAttribute(&g_walk_sms, cudaDevAttrMultiProcessorCount, dev));
+    }
+    const int W = 2 * d.n + 1;
+    // the flag and the bits behind it
+    PS_CUDA(cudaMemsetAsync(d.bad, 0, kWalkCtlBytes + (size_t)W * 2 * (size_t)d.nw * sizeof(uint64_t), st));
+    const int64_t chunks = (int64_t)d.n * (d.w / 2), nblk = (chunks + 256 * kGatherUnroll - 1) / (256 * kGatherUnroll);
+    const int64_t blocks = std::min<int64_t>(W * nblk, (int64_t)g_walk_sms * 4);
+    walk_gather_kernel<<<(unsigned)blocks, 256, 0, st>>>(X, Z, d.n, W, d.w, reinterpret_cast<uint32_t *>(d.gin), d.nw,
+                                                         d.bad, d.rp);
+    PS_CUDA(cudaGetLastError());
+    return OK;
+}
+
+int launch_walk(cudaStream_t st, const WalkDev &d, bool reset, cudaGraphConditionalHandle fall) {
+    const int rc = allow_max_smem((const void *)walk_kernel);
+    if (rc != OK) return rc;
+    walk_kernel<<<1, kWalkThreads, walk_smem_bytes(d.n), st>>>(d, reset ? 1 : 0, fall);
+    PS_CUDA(cudaGetLastError());
+    return OK;
+}
+
+int launch_walk_signs(cudaStream_t st, const WalkDev &d, bool reset) {
+    walk_signs_kernel<<<(unsigned)d.w, kSignThreads, (size_t)(2 * d.n + 1) * sizeof(u64), st>>>(d, reset ? 1 : 0);
+    PS_CUDA(cudaGetLastError());
+    return OK;
+}
+
+}  // namespace ps

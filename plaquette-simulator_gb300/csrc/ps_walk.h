@@ -1,0 +1,108 @@
+// ps_walk.h -- runs on a tableau whose x / z are the same in every shot,
+// with those x / z followed on the device.
+//
+// The argument of ps_frame.h holds from any tableau whose shots share their
+// x / z, not only from |0...0>: under gates, Pauli gates, channels,
+// conditional Paulis and measurements they stay shared, and only the signs
+// are per shot.  From |0...0> the host knows the x / z and compiles a sign
+// program; the walk covers what it does not: runs without reset, whose
+// starting x / z are on the device only, and circuits with conditional
+// Paulis.  Four launches, whatever the circuit's length:
+//   gather     (runs without reset) reads X and Z once, checks that every
+//              (row, qubit) is the same in all shots and keeps one bit of
+//              each; if some are not, the rest of the walk does nothing and
+//              the per-shot kernels that follow in the same run do the work;
+//   walk       one CTA takes that one tableau through the whole circuit in
+//              shared memory and writes down what each step means for the
+//              signs, as bit masks over the tableau rows;
+//   noise      the sign XORs of the channel outcomes (noise_vec_kernel);
+//   signs      one CTA per shot-word applies the masks to its signs, draws
+//              the random outcomes and writes the records;
+// and the final x / z go out to every shot (broadcast_jobs_kernel) beside
+// the last two.
+#pragma once
+#include "ps_internal.h"
+#include "ps_segment.cuh"
+
+namespace ps {
+
+// Registers the walk holds in one CTA's shared memory: up to 511 qubits
+// (a column of 2n + 1 rows is then at most 16 words, half a warp).
+constexpr int64_t kWalkMaxQubits = 511;
+
+// Ops on global qubits, one word each (a thread holds a layer's ops a step
+// ahead of their use):
+//   gate     a | b << 9 | op code << 18
+//   sign op  a | code << 9 | k << 15: code an op code, or kWalkRecX /
+//            kWalkRecZ, the record op r0 + k of the layer
+//   channel  a | b << 16, b = 0xFFFF for a one-qubit channel
+constexpr uint32_t kWalkRecX = 32, kWalkRecZ = 33;
+constexpr uint32_t kWalkMaxRecOps = 1u << 17;  // of a layer
+__host__ __device__ inline uint32_t walk_gate(uint32_t a, uint32_t b, uint32_t code) { return a | b << 9 | code << 18; }
+__host__ __device__ inline uint32_t walk_sign(uint32_t a, uint32_t code, uint32_t k) { return a | code << 9 | k << 15; }
+// A layer of a segment (gates on disjoint qubits, then sign ops and
+// channels that read them), or a measurement phase.
+struct WalkStep {
+    int32_t phase;              // 1: measurements [i0, i1)
+    int32_t i0, i1;             // gates of a layer
+    int32_t s0, s1, n0, n1;     // sign ops, channels
+    int32_t r0;                 // its first record op
+};
+// What the sign kernel does for one segment and the phase after it: noise
+// vector nv (-1: none), record ops [r0, r1), measurements [m0, m1).
+struct WalkPart {
+    int32_t nv, r0, r1, m0, m1;
+};
+// mq[m]: the measurement's qubit, kWalkReset when it resets it, kWalkBreak
+// when an earlier measurement of its phase has reset that qubit (a run of
+// deterministic measurements reads every sign before its resets flip any,
+// which is the program order only while their qubits differ).
+constexpr int32_t kWalkReset = 1 << 30, kWalkBreak = 1 << 29, kWalkQubit = (1 << 29) - 1;
+
+// The walk's word on measurement m: info bit 0 random, bit 1 the outcome's
+// constant, bit 2 reset, from bit 8 the pivot; end: where its run of
+// deterministic measurements ends, or how many rows a random one multiplies.
+struct WalkMeas {
+    uint32_t info;
+    int32_t end;
+};
+
+struct WalkDev {
+    int32_t n, ww, nw;  // qubits, words of a column of 2n + 1 rows, words of a row
+    int32_t nsteps, nparts, nm;
+    int64_t w;
+    const WalkStep *steps;
+    const WalkPart *parts;
+    const uint32_t *gates, *signs, *slots;
+    const int32_t *mq;
+    const int32_t *rec_of_op;  // record op -> circuit record
+    const MeasOp *meas;
+    const RunParams *rp;
+    u64 *rec;     // records: results [nm][w], determined [nm][w]
+    u64 *R;
+    const u64 *nvec;  // noise vectors [nv][w][wp_noise]
+    int64_t nvec_rows;
+    // written by the gather and the walk
+    int32_t *bad;   // not 0: x / z differ between shots (or may not be a valid tableau)
+    uint64_t *gin;  // the gathered bits [2n+1][2][nw]
+    u64 *smask;     // [channel][4][ww]: rows with z(a), x(a), z(b), x(b)
+    u64 *rmask;     // [record op][ww]: the rows it flips
+    WalkMeas *minfo;
+    u64 *mmask;     // [measurement][2][ww]: rows read (by destabilizer); rows that its reset flips
+    uint16_t *mlist;  // [measurement][list_stride]: a random one's multiplied rows, constant in bit 15
+    int64_t list_stride;
+    u64 *fmask;     // [ww] constant flips pending at the end
+    uint64_t *xz;   // final bits [2n+1][2][nw]
+};
+
+// The block of `bad`, in front of gin: the flag, the broadcast's counters.
+constexpr size_t kWalkCtlBytes = 256;
+
+size_t walk_smem_bytes(int64_t n);
+int launch_walk_gather(cudaStream_t st, const u64 *X, const u64 *Z, const WalkDev &d);
+// fall: the condition of the captured graph's per-shot part, set when the
+// walk does not run (0: none).
+int launch_walk(cudaStream_t st, const WalkDev &d, bool reset, cudaGraphConditionalHandle fall);
+int launch_walk_signs(cudaStream_t st, const WalkDev &d, bool reset);
+
+}  // namespace ps
