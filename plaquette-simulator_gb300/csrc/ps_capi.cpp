@@ -107,7 +107,7 @@ int measure_one(ps_state *h, int64_t q, float bias, int64_t id, const uint8_t *f
     op.forced = dforced;
     op.res = rec.res;
     op.det = rec.det;
-    if (h->n > 0 && h->S > 0) TRY(launch_measure(h, &op, 1));
+    if (h->n > 0 && h->S > 0) TRY(launch_measure(h, op));
     if (out_id) *out_id = (uint64_t)rid;
     return OK;
 }

@@ -174,7 +174,6 @@ struct ps_circuit {
     uint32_t *d_psurv = nullptr;    // plain form: survival products of each distinct table, 64 words each
     std::vector<ChannelEst> pest;   // plain form: estimate factors of each distinct table
     u64 **d_recs = nullptr;
-    u64 *d_masks = nullptr;         // plain-mode channel masks (4w)
     u64 *d_forced = nullptr;        // [nm][w]
     NoiseEntry *d_entries = nullptr;
     u64 *d_dense = nullptr;
@@ -2011,9 +2010,6 @@ ps_status ps_circuit_compile(ps_state *h, const ps_op *ops_in, uint64_t nops, co
         if (dev_alloc(h, &p, sizeof(RunParams)) != OK) return bail(E_NOMEM);
         c->owned.push_back(p);
         c->d_params = (RunParams *)p;
-        if (dev_alloc(h, &p, 4 * (size_t)h->w * sizeof(u64)) != OK) return bail(E_NOMEM);
-        c->owned.push_back(p);
-        c->d_masks = (u64 *)p;
     }
 
     // ---- plan (from the cache when this circuit was compiled before)

@@ -309,6 +309,18 @@ PS_HD void phase_add(u64 &c1, u64 &c0, u64 d1, u64 d0) {
     c0 ^= d0;
 }
 
+#ifdef __CUDACC__
+// In a kernel launched by launch_chained: lets the next such kernel be set
+// up, and waits for everything before this one on the stream.  (Without that
+// launch, both do nothing.)
+__device__ __forceinline__ void grid_dependency_wait() {
+#ifdef __CUDA_ARCH__
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
+#endif
+
 // ------------------------------------------------------------- errors
 enum Status : int {
     OK = 0,

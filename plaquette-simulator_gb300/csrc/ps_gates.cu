@@ -61,6 +61,7 @@ template <int CODE>
 __global__ void __launch_bounds__(256) gate1_kernel(u64 *__restrict__ X, u64 *__restrict__ Z, u64 *__restrict__ R,
                                                    int64_t n, int64_t W, int64_t w, int64_t q,
                                                    const u64 *__restrict__ flag) {
+    grid_dependency_wait();
     const int64_t half = w >> 1;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= W * half) return;
@@ -86,6 +87,7 @@ __global__ void __launch_bounds__(256) gate1_kernel(u64 *__restrict__ X, u64 *__
 template <int CODE>
 __global__ void __launch_bounds__(256) gate2_kernel(u64 *__restrict__ X, u64 *__restrict__ Z, u64 *__restrict__ R,
                                                    int64_t n, int64_t W, int64_t w, int64_t c, int64_t t) {
+    grid_dependency_wait();
     const int64_t half = w >> 1;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= W * half) return;
@@ -106,7 +108,7 @@ __global__ void __launch_bounds__(256) gate2_kernel(u64 *__restrict__ X, u64 *__
     st2(R + i * w + k, r.a, r.b);
 }
 
-// Pauli-channel sampling: one thread per shot-word draws the word's
+// Pauli-channel sampling (ps_pauli_channel_1_noalloc): one thread per shot-word draws the word's
 // outcomes (channel_word) and writes its masks: fx = shots with X or Y,
 // fz = Y or Z, for qubit a (masks[0..w), [w..2w)) and b ([2w..3w), [3w..4w)).
 __global__ void __launch_bounds__(256) channel_sample_kernel(u64 *__restrict__ masks, int64_t w, uint64_t seed_arg,
@@ -144,26 +146,22 @@ __global__ void __launch_bounds__(256) sign_flip_kernel(const u64 *__restrict__ 
     st2(R + i * w + k, r.a, r.b);
 }
 
-// The per-op channel of compiled plain runs in one launch: a CTA takes 8
-// shot-words and a block of 64 rows, samples the words first
-// (channel_word_est: the same draws as every other form; threads 0..7; the
-// CTAs of other row blocks draw the same), then flips their signs over its
-// rows, two words a thread (16-byte accesses, four threads a row).
+// A channel in one launch: a CTA takes 8 shot-words and a block of 64 rows,
+// samples the words first (channel_word_est: the same draws as every other
+// form; threads 0..7; the CTAs of other row blocks draw the same), then
+// flips their signs over its rows, two words a thread (16-byte accesses,
+// four threads a row).
 template <int TWO>
-__global__ void __launch_bounds__(256) channel_apply_kernel(const u64 *__restrict__ X, const u64 *__restrict__ Z,
-                                                           u64 *__restrict__ R, int64_t n, int64_t W, int64_t w,
-                                                           int64_t a, int64_t b, uint32_t event_off,
-                                                           const RunParams *__restrict__ rp,
-                                                           const uint64_t *__restrict__ thr, int count,
-                                                           const uint32_t *__restrict__ surv, ChannelEst est) {
+__device__ __forceinline__ void channel_apply(const u64 *__restrict__ X, const u64 *__restrict__ Z, u64 *__restrict__ R,
+                                              int64_t n, int64_t W, int64_t w, int64_t a, int64_t b, uint64_t seed,
+                                              uint64_t event, uint64_t word_base, const uint64_t *thr, int count,
+                                              const uint32_t *surv, ChannelEst est) {
     __shared__ u64 sm[4][8];
     const int64_t k0 = (int64_t)blockIdx.x * 8;
     const int t = threadIdx.x;
     if (t < 8) {
         ChannelWord m{0ull, 0ull, 0ull, 0ull};
-        if (k0 + t < w)
-            m = channel_word_est(rp->seed, rp->event_base + event_off, rp->word_base + (uint64_t)(k0 + t), thr, count,
-                                 surv, est);
+        if (k0 + t < w) m = channel_word_est(seed, event, word_base + (uint64_t)(k0 + t), thr, count, surv, est);
         sm[0][t] = m.fxa;
         sm[1][t] = m.fza;
         sm[2][t] = m.fxb;
@@ -191,48 +189,80 @@ __global__ void __launch_bounds__(256) channel_apply_kernel(const u64 *__restric
     }
 }
 
+// In compiled plain runs the channel's table is on the device and the run's
+// parameters too.
+template <int TWO>
+__global__ void __launch_bounds__(256) channel_apply_kernel(const u64 *__restrict__ X, const u64 *__restrict__ Z,
+                                                           u64 *__restrict__ R, int64_t n, int64_t W, int64_t w,
+                                                           int64_t a, int64_t b, uint32_t event_off,
+                                                           const RunParams *__restrict__ rp,
+                                                           const uint64_t *__restrict__ thr, int count,
+                                                           const uint32_t *__restrict__ surv, ChannelEst est) {
+    channel_apply<TWO>(X, Z, R, n, W, w, a, b, rp->seed, rp->event_base + event_off, rp->word_base, thr, count, surv,
+                       est);
+}
+
+// In the op-by-op API the table travels as a kernel argument: no copy, no
+// allocation, one launch (97 qubits, 20,000 shots: 5 us a channel; sampling
+// and flip launches with an allocation and a copy around them took 16 to 20).
+struct ChannelTable {
+    uint64_t thr[16];
+    uint32_t surv[64];
+    ChannelEst est;
+};
+template <int TWO>
+__global__ void __launch_bounds__(256) channel_op_kernel(const u64 *__restrict__ X, const u64 *__restrict__ Z,
+                                                        u64 *__restrict__ R, int64_t n, int64_t W, int64_t w, int64_t a,
+                                                        int64_t b, uint64_t seed, uint64_t event, uint64_t word_base,
+                                                        int count, const __grid_constant__ ChannelTable t) {
+    grid_dependency_wait();
+    channel_apply<TWO>(X, Z, R, n, W, w, a, b, seed, event, word_base, t.thr, count, t.surv, t.est);
+}
+
 inline int blocks_for(int64_t threads) { return (int)((threads + 255) / 256); }
 
 }  // namespace
 
-int launch_gate_on(cudaStream_t st, ps_state *h, int32_t code, int64_t a, int64_t b, const u64 *flag) {
+namespace {
+// chained: a call of the op-by-op API (launch_chained), else a launch as it
+// is captured in a plain circuit's graph.
+template <class... P, class... A>
+void gate_launch(bool chained, cudaStream_t st, int grid, void (*kernel)(P...), A... args) {
+    if (chained)
+        (void)launch_chained(st, dim3((unsigned)grid), dim3(256), 0, kernel, args...);  // (its error: cudaGetLastError)
+    else
+        kernel<<<grid, 256, 0, st>>>(args...);
+}
+
+int launch_gate_as(bool chained, cudaStream_t st, ps_state *h, int32_t code, int64_t a, int64_t b, const u64 *flag) {
     const int64_t work = h->W * (h->w >> 1);
     const int grid = blocks_for(work);
     if (h->n == 0 || work == 0) return OK;
+    auto one = [&](auto kernel) { gate_launch(chained, st, grid, kernel, h->X, h->Z, h->R, h->n, h->W, h->w, a, flag); };
+    auto two = [&](auto kernel) { gate_launch(chained, st, grid, kernel, h->X, h->Z, h->R, h->n, h->W, h->w, a, b); };
     switch (code) {
-    case OP_H: gate1_kernel<OP_H><<<grid, 256, 0, st>>>(h->X, h->Z, h->R, h->n, h->W, h->w, a, nullptr); break;
-    case OP_S: gate1_kernel<OP_S><<<grid, 256, 0, st>>>(h->X, h->Z, h->R, h->n, h->W, h->w, a, nullptr); break;
-    case OP_X: gate1_kernel<OP_X><<<grid, 256, 0, st>>>(h->X, h->Z, h->R, h->n, h->W, h->w, a, nullptr); break;
-    case OP_Y: gate1_kernel<OP_Y><<<grid, 256, 0, st>>>(h->X, h->Z, h->R, h->n, h->W, h->w, a, nullptr); break;
-    case OP_Z: gate1_kernel<OP_Z><<<grid, 256, 0, st>>>(h->X, h->Z, h->R, h->n, h->W, h->w, a, nullptr); break;
-    case OP_H_IF: gate1_kernel<OP_H_IF><<<grid, 256, 0, st>>>(h->X, h->Z, h->R, h->n, h->W, h->w, a, flag); break;
-    case OP_S_IF: gate1_kernel<OP_S_IF><<<grid, 256, 0, st>>>(h->X, h->Z, h->R, h->n, h->W, h->w, a, flag); break;
-    case OP_CX: gate2_kernel<OP_CX><<<grid, 256, 0, st>>>(h->X, h->Z, h->R, h->n, h->W, h->w, a, b); break;
-    case OP_CZ: gate2_kernel<OP_CZ><<<grid, 256, 0, st>>>(h->X, h->Z, h->R, h->n, h->W, h->w, a, b); break;
+    case OP_H: one(gate1_kernel<OP_H>); break;
+    case OP_S: one(gate1_kernel<OP_S>); break;
+    case OP_X: one(gate1_kernel<OP_X>); break;
+    case OP_Y: one(gate1_kernel<OP_Y>); break;
+    case OP_Z: one(gate1_kernel<OP_Z>); break;
+    case OP_H_IF: one(gate1_kernel<OP_H_IF>); break;
+    case OP_S_IF: one(gate1_kernel<OP_S_IF>); break;
+    case OP_CX: two(gate2_kernel<OP_CX>); break;
+    case OP_CZ: two(gate2_kernel<OP_CZ>); break;
     default: return fail(E_ARG, "unknown gate code " + std::to_string(code));
     }
     PS_CUDA(cudaGetLastError());
     return OK;
 }
+}  // namespace
 
-int launch_gate(ps_state *h, int32_t code, int64_t a, int64_t b, const u64 *flag) {
-    return launch_gate_on(h->stream, h, code, a, b, flag);
+int launch_gate_on(cudaStream_t st, ps_state *h, int32_t code, int64_t a, int64_t b, const u64 *flag) {
+    return launch_gate_as(false, st, h, code, a, b, flag);
 }
 
-int launch_channel_rp(cudaStream_t st, ps_state *h, int64_t a, int64_t b, const uint64_t *dev_thr, int count,
-                      uint32_t event_off, const RunParams *rp, u64 *masks) {
-    channel_sample_kernel<<<blocks_for(h->w), 256, 0, st>>>(masks, h->w, (uint64_t)h->seed, event_off, (uint64_t)h->word_base, rp, count,
-                                                             dev_thr);
-    PS_CUDA(cudaGetLastError());
-    const int64_t work = h->W * (h->w >> 1);
-    if (h->n > 0 && work > 0) {
-        sign_flip_kernel<<<blocks_for(work), 256, 0, st>>>(h->X, h->Z, h->R, h->n, h->W, h->w, a, masks, masks + h->w);
-        if (count == 15)
-            sign_flip_kernel<<<blocks_for(work), 256, 0, st>>>(h->X, h->Z, h->R, h->n, h->W, h->w, b,
-                                                                masks + 2 * h->w, masks + 3 * h->w);
-    }
-    PS_CUDA(cudaGetLastError());
-    return OK;
+int launch_gate(ps_state *h, int32_t code, int64_t a, int64_t b, const u64 *flag) {
+    return launch_gate_as(true, h->stream, h, code, a, b, flag);
 }
 
 int launch_channel_apply(cudaStream_t st, ps_state *h, int64_t a, int64_t b, const uint64_t *dev_thr, int count,
@@ -272,22 +302,15 @@ void channel_thresholds(const float *p, int count, uint64_t *thr) {
 
 int launch_pauli_channel(ps_state *h, int64_t a, int64_t b, const uint64_t *thr, int count) {
     const uint64_t event = h->events++;
-    uint64_t *dthr = nullptr;
-    PS_CUDA(cudaMallocAsync(&dthr, 16 * sizeof(uint64_t), h->stream));
-    PS_CUDA(cudaMemcpyAsync(dthr, thr, (size_t)(count + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, h->stream));
-    channel_sample_kernel<<<blocks_for(h->w), 256, 0, h->stream>>>(h->mask_buf, h->w, (uint64_t)h->seed, event, (uint64_t)h->word_base,
-                                                                    nullptr, count, dthr);
-    PS_CUDA(cudaGetLastError());
-    const int64_t work = h->W * (h->w >> 1);
-    if (h->n > 0 && work > 0) {
-        sign_flip_kernel<<<blocks_for(work), 256, 0, h->stream>>>(h->X, h->Z, h->R, h->n, h->W, h->w, a, h->mask_buf,
-                                                                  h->mask_buf + h->w);
-        if (count == 15)
-            sign_flip_kernel<<<blocks_for(work), 256, 0, h->stream>>>(h->X, h->Z, h->R, h->n, h->W, h->w, b,
-                                                                      h->mask_buf + 2 * h->w, h->mask_buf + 3 * h->w);
-    }
-    PS_CUDA(cudaGetLastError());
-    PS_CUDA(cudaFreeAsync(dthr, h->stream));
+    if (h->n == 0 || h->w == 0) return OK;
+    ChannelTable t;
+    for (int k = 0; k <= count; ++k) t.thr[k] = thr[k];
+    channel_surv_table(thr[count - 1], t.surv);
+    t.est = channel_est_factors(thr[count - 1], count);
+    const dim3 grid((unsigned)((h->w + 7) / 8), (unsigned)((h->W + 63) / 64));
+    const uint64_t seed = (uint64_t)h->seed, word_base = (uint64_t)h->word_base;
+    PS_CUDA(launch_chained(h->stream, grid, dim3(256), 0, count == 15 ? channel_op_kernel<1> : channel_op_kernel<0>, h->X,
+                           h->Z, h->R, h->n, h->W, h->w, a, b, seed, event, word_base, count, t));
     return OK;
 }
 

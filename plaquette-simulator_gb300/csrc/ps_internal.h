@@ -88,9 +88,6 @@ struct ps_state {
     cudaStream_t stream = nullptr;
     // Device scratch for single-op calls.
     u64 *forced_buf = nullptr;   // w words
-    u64 *mask_buf = nullptr;     // 4*w words (Pauli-channel masks)
-    ps::MeasOp *meas_buf = nullptr;
-    size_t meas_cap = 0;
     std::vector<ps::Record> recs;
     ps::RecordArena arena;
     int device = 0;
@@ -121,6 +118,26 @@ struct NvtxRange {
 
 // ps_capi.cpp: records the entry point for error messages, clears the error.
 void ps_enter(const char *method, int line);
+
+// Launches a kernel whose first act is grid_dependency_wait() so that it may
+// be set up while the kernel before it on the stream still runs
+// (programmatic stream serialisation).  A program that calls gate by gate is
+// a chain of launches of a few microseconds; back to back they came every
+// 4.1 us, set up early every 2.3 (the host's own time a call).
+template <class... P, class... A>
+inline cudaError_t launch_chained(cudaStream_t st, dim3 grid, dim3 block, size_t smem, void (*kernel)(P...), A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 // ps_state.cu
 // Device memory of a state and of everything compiled for it.
@@ -160,7 +177,7 @@ int check_channel_probs(const float *p, int count);
 
 // ps_measure.cu
 struct RunParams;
-int launch_measure(ps_state *h, const MeasOp *ops_host, int nops);
+int launch_measure(ps_state *h, const MeasOp &op);  // one measurement, on the state's stream
 // words_per_cta: 1, 2 or 4 shot-words per CTA, 0 = automatic.
 // bad (here and below): a device word, null or not 0 for the launch to do
 // its work; 0 when another plan of the same run has done it (ps_walk.h).
@@ -192,8 +209,6 @@ constexpr size_t kFrameStageMax = 100 * 1024;
 // flips); dev_surv: its table's survival products (channel_surv_table).
 int launch_channel_apply(cudaStream_t st, ps_state *h, int64_t a, int64_t b, const uint64_t *dev_thr, int count,
                          const uint32_t *dev_surv, ChannelEst est, uint32_t event_off, const RunParams *rp);
-int launch_channel_rp(cudaStream_t stream, ps_state *h, int64_t a, int64_t b, const uint64_t *dev_thr, int count,
-                      uint32_t event_off, const RunParams *rp, u64 *dev_masks);
 int launch_gate_on(cudaStream_t stream, ps_state *h, int32_t code, int64_t a, int64_t b, const u64 *flag);
 } // namespace ps
 

@@ -16,6 +16,7 @@ namespace {
 // z(i,j)=[i-n==j], r(i)=[i==2n], for every shot (all 64 bits of a word).
 __global__ void init_zero_kernel(u64 *__restrict__ X, u64 *__restrict__ Z, u64 *__restrict__ R, int64_t n, int64_t W,
                                  int64_t w) {
+    grid_dependency_wait();
     const int64_t cells = W * n * w;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < cells; idx += stride) {
@@ -175,11 +176,9 @@ int state_alloc(ps_state *h, int64_t n, int64_t S, int64_t seed, DevPool *pool, 
     h->X = (u64 *)px;
     h->Z = (u64 *)pz;
     h->R = (u64 *)pr;
-    void *pf = nullptr, *pm = nullptr;
+    void *pf = nullptr;
     if (dev_alloc(h, &pf, (size_t)w * sizeof(u64)) != OK) return E_NOMEM;
     h->forced_buf = (u64 *)pf;
-    if (dev_alloc(h, &pm, (size_t)4 * w * sizeof(u64)) != OK) return E_NOMEM;
-    h->mask_buf = (u64 *)pm;
     h->arena.words = (size_t)w;
     return OK;
 }
@@ -190,7 +189,7 @@ size_t state_bytes(int64_t n, int64_t S, bool signs_only) {
     w = (w + 1) & ~int64_t(1);
     if (w == 0) w = 2;
     const size_t W = 2 * (size_t)n + 1;
-    return (signs_only ? 0 : 2 * W * (size_t)(n > 0 ? n : 1) * (size_t)w * 8) + W * (size_t)w * 8 + 5 * (size_t)w * 8;
+    return (signs_only ? 0 : 2 * W * (size_t)(n > 0 ? n : 1) * (size_t)w * 8) + W * (size_t)w * 8 + (size_t)w * 8;
 }
 
 void state_free(ps_state *h) {
@@ -199,16 +198,13 @@ void state_free(ps_state *h) {
     dev_free(h, h->Z);
     dev_free(h, h->R);
     dev_free(h, h->forced_buf);
-    dev_free(h, h->mask_buf);
-    dev_free(h, h->meas_buf);
     for (u64 *c : h->arena.chunks) dev_free(h, c);
     for (u64 *c : h->arena.blocks) dev_free(h, c);
     h->arena.chunks.clear();
     h->arena.blocks.clear();
     if (h->stream) cudaStreamDestroy(h->stream);
     h->X = h->Z = h->R = nullptr;
-    h->forced_buf = h->mask_buf = nullptr;
-    h->meas_buf = nullptr;
+    h->forced_buf = nullptr;
 }
 
 int launch_init_zero_on(cudaStream_t stream, ps_state *h) {
@@ -218,7 +214,12 @@ int launch_init_zero_on(cudaStream_t stream, ps_state *h) {
     return OK;
 }
 
-int launch_init_zero(ps_state *h) { return launch_init_zero_on(h->stream, h); }
+int launch_init_zero(ps_state *h) {
+    if (h->n == 0) return OK;
+    PS_CUDA(launch_chained(h->stream, dim3((unsigned)grid_for(h->W * h->n * h->w)), dim3(256), 0, init_zero_kernel, h->X,
+                           h->Z, h->R, h->n, h->W, h->w));
+    return OK;
+}
 
 int record_new(ps_state *h, int64_t q, int64_t *id) {
     RecordArena &a = h->arena;
