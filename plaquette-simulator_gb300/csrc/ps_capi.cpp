@@ -537,6 +537,7 @@ ps_status ps_get_record_device(ps_state *h, uint64_t id, void **results, void **
     ENTER();
     CHECK_HANDLE(h);
     if (id >= h->recs.size()) return fail(E_RANGE, "Measurement id is out of range.");
+    h->recs[(size_t)id].exposed = true;
     if (results) *results = h->recs[(size_t)id].res;
     if (determined) *determined = h->recs[(size_t)id].det;
     return OK;

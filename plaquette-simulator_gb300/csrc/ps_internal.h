@@ -25,6 +25,7 @@ struct Record {
     u64 *det = nullptr;  // device, w words
     std::vector<u64> host_res, host_det;
     bool host_valid = false;
+    bool exposed = false;  // its device words were handed out (ps_get_record_device)
 };
 
 // Pool of fixed-size device blocks for records (one cudaMalloc per 64
@@ -89,6 +90,7 @@ struct ps_state {
     // Device scratch for single-op calls.
     u64 *forced_buf = nullptr;   // w words
     std::vector<ps::Record> recs;
+    std::vector<u64> rec_host;   // staging of record_fetch
     ps::RecordArena arena;
     int device = 0;
     // True while the tableau is known to be a valid stabilizer tableau

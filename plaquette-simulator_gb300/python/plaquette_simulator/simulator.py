@@ -16,11 +16,13 @@ import numpy as np
 from . import _lib
 from ._lib import PS_E_RANGE, PlaquetteError, check
 
-_vp = C.c_void_p
-
 
 def _ptr(a: Optional[np.ndarray]):
-    return None if a is None else a.ctypes.data_as(_vp)
+    """The array's address for the length of a call (the caller holds the array)."""
+    return None if a is None else a.ctypes.data
+
+
+_F3, _F15 = C.c_float * 3, C.c_float * 15
 
 
 def _forced_bytes(forced, batch: int) -> Optional[np.ndarray]:
@@ -191,10 +193,16 @@ class CliffordState:
         return out.value
 
     def pauli_channel_1(self, q: int, px: float, py: float, pz: float) -> None:
+        if type(px) is type(py) is type(pz) is float:
+            check(self._L.ps_pauli_channel_1(self._h, q, _F3(px, py, pz)))
+            return
         p = np.asarray([px, py, pz], dtype=np.float32)
         check(self._L.ps_pauli_channel_1(self._h, q, _ptr(p)))
 
     def pauli_channel_2(self, a: int, b: int, probs: Sequence[float]) -> None:
+        if type(probs) in (list, tuple) and len(probs) == 15 and set(map(type, probs)) == {float}:
+            check(self._L.ps_pauli_channel_2(self._h, a, b, _F15(*probs)))
+            return
         p = np.ascontiguousarray(probs, dtype=np.float32)
         if p.size != 15:
             raise ValueError("15 probabilities required")
@@ -228,8 +236,8 @@ class CliffordState:
     def record_bits(self, measurement_id: int) -> Tuple[np.ndarray, np.ndarray]:
         """Packed result / determined bits of one record (LSB-first bytes)."""
         nb = (self._batch + 7) // 8
-        res = np.zeros(nb, dtype=np.uint8)
-        det = np.zeros(nb, dtype=np.uint8)
+        res = np.empty(nb, dtype=np.uint8)
+        det = np.empty(nb, dtype=np.uint8)
         check(self._L.ps_get_record_bits(self._h, measurement_id, _ptr(res), _ptr(det)))
         return res, det
 

@@ -1,0 +1,76 @@
+"""Record reads bring along the unread records next to them: reads in any
+order, between measurements into old and new records, across chunks of 64
+records, and beside records whose device words a caller writes itself, always
+give what the device holds."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shots", [1, 700, 200000])
+def test_reads_between_measurements(ps, O, shots):
+    n = 3
+    st, o = ps.CliffordState(n, shots, 5, True), O.Oracle(n, shots, seed=5)
+    ops = {"h": 0, "cx": 5, "m": 7}
+
+    def both(name, a, b=0):
+        o.run(np.array([(ops[name], a, b, -1)], np.int32), np.zeros(1, np.float32))
+
+    def same(k):
+        res, det = st.record(k)
+        ores, odet = o.record(k)
+        assert np.array_equal(res, ores) and np.array_equal(det, odet), k
+
+    count = 0
+    for step in range(70 if shots < 1000 else 12):
+        st.apply_hadamard_gate(step % n)
+        both("h", step % n)
+        st.apply_control_not_gate(step % n, (step + 1) % n)
+        both("cx", step % n, (step + 1) % n)
+        for q in range(n):
+            st.measure_qubit(q)
+            both("m", q)
+        count += n
+        if step % 5 == 3:
+            for k in (count - 2, 0, count // 2, count - 1):
+                same(k)
+    for k in (count - 1, 63, 64, 65, 1, count // 2):
+        if k < count:
+            same(k)
+    # into an old record whose neighbours are read already, then all of them again
+    st.measure_qubit(1, measurement_id=4, forced=np.zeros(shots, np.uint8))
+    before = st.record(4)[0].copy()
+    st.apply_pauli_x_gate(1)
+    st.measure_qubit(1, measurement_id=4)
+    assert np.array_equal(st.record(4)[0], 1 - before)
+    for k in range(count):
+        if k != 4:
+            same(k)
+
+
+@pytest.mark.gpu
+def test_records_written_by_the_caller(ps):
+    from plaquette_simulator import _lib
+    L = _lib.load()
+    st = ps.CliffordState(2, 64, 5, True)
+    ids = [st.measure_qubit(0) for _ in range(4)]
+    assert ids == [0, 1, 2, 3]
+    st.measure_qubit(0, measurement_id=3)
+    r, d = C.c_void_p(), C.c_void_p()
+    _lib.check(L.ps_get_record_device(st.handle, 2, C.byref(r), C.byref(d)))
+    src, sd = C.c_void_p(), C.c_void_p()
+    st.apply_pauli_x_gate(0)
+    st.measure_qubit(0, measurement_id=0)  # all ones
+    _lib.check(L.ps_get_record_device(st.handle, 0, C.byref(src), C.byref(sd)))
+    assert not st.record(1)[0].any() and not st.record(3)[0].any()  # their neighbour 2 stays unread
+    import torch
+
+    class Words:
+        def __init__(self, p):
+            self.__cuda_array_interface__ = {"shape": (2,), "typestr": "<i8", "data": (p, False), "version": 3}
+    st.synchronize()
+    torch.as_tensor(Words(r.value), device="cuda").copy_(torch.as_tensor(Words(src.value), device="cuda"))
+    torch.cuda.synchronize()
+    assert st.record(2)[0].all() and st.record(0)[0].all()
