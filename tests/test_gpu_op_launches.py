@@ -58,3 +58,43 @@ def test_ops_back_to_back_match_oracle(ps, O, n, shots):
         res, det = st.record(r)
         ores, odet = o.record(r)
         assert np.array_equal(res, ores) and np.array_equal(det, odet), r
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 100, 128, 129, 256, 300])
+@pytest.mark.parametrize("words", [152, 154, 306, 612])
+def test_measurements_of_wide_states_equal_narrow_ones(ps, n, words):
+    """Wide states measure with fewer threads a shot-word: every shot-word
+    ends as in a narrow state that holds only those shots."""
+    from plaquette_simulator import circuits as C
+    shots = 64 * words - 7
+    rng = C.SplitMix64(n + words)
+    ops = [(rng.below(6), rng.below(n), rng.below(n)) for _ in range(60)]
+
+    def run(st):
+        rec = []
+        for kind, a, b in ops:
+            if kind < 2:
+                st.apply_hadamard_gate(a)
+            elif kind == 2 and a != b:
+                st.apply_control_not_gate(a, b)
+            elif kind == 3:
+                st.apply_phase_gate(a)
+            elif kind == 4:
+                rec.append(st.measure_qubit(a, 0.3))
+            else:
+                rec.append(st.reset_qubit(a))
+        return [np.concatenate([st.record(r)[0], st.record(r)[1]]) for r in rec]
+
+    wide = ps.CliffordState(n, shots, 13, True)
+    recs = run(wide)
+    for first, count in ((0, 2), (words // 2 & ~1, 2), (words - 2, 2)):
+        k = min(64 * count, shots - 64 * first)
+        narrow = ps.CliffordState(n, k, 13, True)
+        narrow.set_shot_offset(64 * first)
+        nrec = run(narrow)
+        for u, v in zip(wide.tableau_words(first, count), narrow.tableau_words(0, count)):
+            assert np.array_equal(u, v)
+        for u, v in zip(recs, nrec):
+            assert np.array_equal(u[:shots][64 * first:64 * first + k], v[:k])
+            assert np.array_equal(u[shots:][64 * first:64 * first + k], v[k:])
