@@ -198,6 +198,7 @@ struct ps_circuit {
     FrameProgram fprog;
     FrameOp *d_fops = nullptr;
     uint32_t *d_ftab = nullptr;
+    uint16_t *d_fnrows = nullptr;
     int32_t *d_frand = nullptr;
     uint64_t *d_fxz = nullptr;
     // The shared-x/z plan as a job table of one job (ps_frame_dev.h): one
@@ -1041,16 +1042,14 @@ int enqueue_steps(ps_circuit *c, cudaStream_t st, size_t from, size_t to, Profil
 // from global memory.  E_ARG: the program does not fit this kernel (the
 // per-shot plan runs instead).
 int frame_job_ranges(ps_circuit *c, const FrameProgram &P, FrameJobDev &job, std::vector<FrameRangeDev> &ranges,
-                     std::vector<FrameSlotDev> &slots, std::vector<uint32_t> &s64, std::vector<uint32_t> &events,
-                     std::vector<int32_t> &nv_range, std::vector<FrameChanTab> &ctabs,
+                     std::vector<FrameSlotDev> &slots, std::vector<uint32_t> &s64, std::vector<int32_t> &nv_range, std::vector<FrameChanTab> &ctabs,
                      std::vector<uint32_t> &surv) {
     ps_state *h = c->h;
     ranges.clear();
     uint32_t max_rand = 0, max_scratch = 0, max_slots = 0;
-    // channel records (indexed like slot_off) and the distinct tables
+    // channel records and the distinct tables
     slots.clear();
     nv_range.clear();
-    events.assign(P.slot_off.size(), 0u);
     s64.clear();
     std::map<int32_t, uint32_t> table_of;
     ctabs.clear();
@@ -1068,18 +1067,24 @@ int frame_job_ranges(ps_circuit *c, const FrameProgram &P, FrameJobDev &job, std
                 return fail(E_ARG, "shared-x/z plan: a sampled range must start with its noise");
             const SegHost &sg = c->segs[(size_t)L.seg];
             r.nslots = (int32_t)sg.slots.size();
-            r.slot_base = (uint32_t)P.ops[L.op0].arg;
+            const size_t slot_base = (size_t)P.ops[L.op0].arg;
             max_slots = std::max(max_slots, (uint32_t)r.nslots);
-            if ((size_t)r.slot_base + (size_t)r.nslots >= events.size())
+            if (slot_base + (size_t)r.nslots >= P.slot_rows.size())
                 return fail(E_ARG, "shared-x/z plan: channel table out of range");
-            // this segment's channel records from a 16-byte boundary, padded to one
             r.rec_base = (uint32_t)slots.size();
-            slots.resize(slots.size() + (((size_t)r.nslots + 1) & ~(size_t)1), FrameSlotDev{0u, kFrameNoHit});
+            slots.resize(slots.size() + (size_t)r.nslots, FrameSlotDev{0u, kFrameNoHit, {}, {}});
             // this segment's S_64 words from a 16-byte boundary, padded to one
             r.s64_base = (uint32_t)s64.size();
             s64.resize(s64.size() + (((size_t)r.nslots + 3) & ~(size_t)3), 0xFFFFFFFFu);
+            // Channels in the order of their events, which are consecutive in a
+            // segment (its slots are in layer order): the kernel draws the
+            // first numbers of four events from one Philox block.
+            r.ev0 = sg.slots.empty() ? 0u : sg.slots[0].event;
+            for (const NoiseSlot &sl : sg.slots) r.ev0 = std::min(r.ev0, sl.event);
             for (int32_t q = 0; q < r.nslots; ++q) {
                 const NoiseSlot &sl = sg.slots[(size_t)q];
+                const size_t at = (size_t)(sl.event - r.ev0);
+                if (at >= (size_t)r.nslots) return fail(E_ARG, "shared-x/z plan: a segment's channel events are not consecutive");
                 auto it = table_of.find(sl.thr_off);
                 if (it == table_of.end()) {
                     if (ctabs.size() >= kFrameMaxTables) return fail(E_ARG, "shared-x/z plan: too many channel tables");
@@ -1093,26 +1098,18 @@ int frame_job_ranges(ps_circuit *c, const FrameProgram &P, FrameJobDev &job, std
                     surv.resize(surv.size() + 64);
                     channel_surv_table(c->thr_host[(size_t)(sl.thr_off + sl.count - 1)], &surv[surv.size() - 64]);
                 }
-                const uint32_t t0 = P.slot_off[(size_t)r.slot_base + (size_t)q];
-                const uint32_t len = P.slot_off[(size_t)r.slot_base + (size_t)q + 1] - t0;
-                if (len > kFrameMaxSlotRows) return fail(E_ARG, "shared-x/z plan: a channel flips too many rows");
                 const bool never = c->thr_host[(size_t)(sl.thr_off + sl.count - 1)] == 0;
-                FrameSlotDev &d = slots[(size_t)r.rec_base + (size_t)q];
-                d.t0 = t0;
-                d.lt = len << 12 | (never ? kFrameNoHit : it->second);
-                events[(size_t)r.slot_base + (size_t)q] = sl.event;
-                s64[(size_t)r.s64_base + (size_t)q] =
+                FrameSlotDev &d = slots[(size_t)r.rec_base + at];
+                const FrameProgram::SlotRows &rows = P.slot_rows[slot_base + (size_t)q];
+                d.t0 = rows.t0;
+                std::memcpy(d.len, rows.len, sizeof d.len);
+                std::memcpy(d.rows, rows.rows, sizeof d.rows);
+                d.table = never ? kFrameNoHit : it->second;
+                s64[(size_t)r.s64_base + at] =
                     never ? 0xFFFFFFFFu : (uint32_t)c->thr_host[(size_t)(sl.thr_off + sl.count)];
             }
         }
-        r.ev0 = -1;
         r.nv = -1;
-        if (r.nslots > 0) {  // consecutive events: the kernel draws first draws four channels a block
-            bool run = true;
-            for (int32_t q = 1; q < r.nslots && run; ++q)
-                run = events[(size_t)r.slot_base + q] == events[(size_t)r.slot_base] + (uint32_t)q;
-            if (run && events[(size_t)r.slot_base] <= 0x7FFFFFFFu) r.ev0 = (int32_t)events[(size_t)r.slot_base];
-        }
         if (r.nslots > 0) {  // its noise vectors: block nv of nvec
             r.nv = (int32_t)nv_range.size();
             nv_range.push_back((int32_t)ranges.size());
@@ -1122,13 +1119,14 @@ int frame_job_ranges(ps_circuit *c, const FrameProgram &P, FrameJobDev &job, std
         ranges.push_back(r);
     }
     if (ranges.empty()) return fail(E_ARG, "shared-x/z plan: empty program");
-    if (slots.empty()) slots.resize(2, FrameSlotDev{0u, kFrameNoHit});
+    if (slots.empty()) slots.push_back(FrameSlotDev{0u, kFrameNoHit, {}, {}});
     if (s64.empty()) s64.resize(4, 0xFFFFFFFFu);
     job.R = h->R;
     job.n = h->n;
     job.w = h->w;
     job.ops = c->d_fops;
     job.tab = c->d_ftab;
+    job.nrows = c->d_fnrows;
     job.nranges = (int32_t)ranges.size();
     job.rand_meas = c->d_frand;
     job.meas = c->d_meas;
@@ -1277,9 +1275,11 @@ int build_walk(ps_circuit *c) {
                 L.op1 = L.op0 + 1;
                 FrameOp op{};
                 op.kind = F_NOISE;
-                op.arg = (int32_t)P.slot_off.size();
+                op.arg = (int32_t)P.slot_rows.size();
                 P.ops.push_back(op);
-                P.slot_off.resize(P.slot_off.size() + sg.slots.size() + 1, 0u);
+                P.slot_rows.resize(P.slot_rows.size() + sg.slots.size() + 1);
+                for (size_t q = 0; q < sg.slots.size(); ++q)  // the channel's place in smask
+                    P.slot_rows[(size_t)op.arg + q].t0 = (uint32_t)(slots.size() - sg.slots.size() + q);
                 P.launches.push_back(L);
             }
         } else if (s.kind == K_MEAS) {
@@ -1367,27 +1367,22 @@ int build_walk(ps_circuit *c) {
         FrameJobDev job{};
         std::vector<FrameRangeDev> ranges;
         std::vector<FrameSlotDev> fslots;
-        std::vector<uint32_t> fs64, fev, surv;
+        std::vector<uint32_t> fs64, surv;
         std::vector<int32_t> nvr;
         std::vector<FrameChanTab> ctabs;
-        int rc = frame_job_ranges(c, P, job, ranges, fslots, fs64, fev, nvr, ctabs, surv);
+        int rc = frame_job_ranges(c, P, job, ranges, fslots, fs64, nvr, ctabs, surv);
         if (rc != OK) return rc;
-        uint32_t ord = 0;  // the channel's place in smask
-        for (const FrameRangeDev &r : ranges)
-            for (int32_t q = 0; q < r.nslots; ++q) fslots[(size_t)r.rec_base + (size_t)q].t0 = ord++;
         FrameRangeDev *dr;
         FrameSlotDev *dfs;
-        uint32_t *ds64, *dev, *dsv;
+        uint32_t *ds64, *dsv;
         FrameChanTab *dct;
         int32_t *dnvr;
         if (upload(h, c->owned, ranges, &dr) || upload(h, c->owned, fslots, &dfs) || upload(h, c->owned, fs64, &ds64) ||
-            upload(h, c->owned, fev, &dev) || upload(h, c->owned, ctabs, &dct) || upload(h, c->owned, surv, &dsv) ||
-            upload(h, c->owned, nvr, &dnvr))
+            upload(h, c->owned, ctabs, &dct) || upload(h, c->owned, surv, &dsv) || upload(h, c->owned, nvr, &dnvr))
             return E_NOMEM;
         job.ranges = dr;
         job.slot = dfs;
         job.slot_s64 = ds64;
-        job.slot_event = dev;
         job.ctab = dct;
         job.surv = dsv;
         job.nv_range = dnvr;
@@ -2165,9 +2160,9 @@ ps_status ps_circuit_compile(ps_state *h, const ps_op *ops_in, uint64_t nops, co
             const size_t fixed = frame_smem_bytes(h->n) + (size_t)h->n * sizeof(u64) + 16;
             fb.linearize(fixed < kSegSmemMax ? (uint32_t)std::min<size_t>((kSegSmemMax - fixed) / sizeof(u64), 1u << 20)
                                              : 0u);
+            fb.prog.pack_noise();
             c->fprog = std::move(fb.prog);
             c->fprog.tab.insert(c->fprog.tab.end(), 4, 0u);  // padding: staged ranges round up to 16 bytes
-            if (c->fprog.slot_off.empty()) c->fprog.slot_off.push_back(0);
             if (c->fprog.rand_meas.empty()) c->fprog.rand_meas.push_back(0);
             if (fresh) {
                 fresh->has_frame = true;
@@ -2177,16 +2172,16 @@ ps_status ps_circuit_compile(ps_state *h, const ps_op *ops_in, uint64_t nops, co
         if (ok) {
             if (upload(h, c->owned, c->fprog.ops, &c->d_fops) || upload(h, c->owned, c->fprog.tab, &c->d_ftab) ||
                 upload(h, c->owned, c->fprog.xz, &c->d_fxz) ||
-                upload(h, c->owned, c->fprog.rand_meas, &c->d_frand))
+                upload(h, c->owned, c->fprog.rand_meas, &c->d_frand) || upload(h, c->owned, c->fprog.nrows, &c->d_fnrows))
                 return bail(E_CUDA);
             FrameJobDev job{};
             std::vector<FrameRangeDev> ranges;
             std::vector<FrameSlotDev> fslots;
-            std::vector<uint32_t> fs64, fev;
+            std::vector<uint32_t> fs64;
             std::vector<int32_t> nvr;
             std::vector<FrameChanTab> ctabs;
             std::vector<uint32_t> surv;
-            const int jrc = frame_job_ranges(c, c->fprog, job, ranges, fslots, fs64, fev, nvr, ctabs, surv);
+            const int jrc = frame_job_ranges(c, c->fprog, job, ranges, fslots, fs64, nvr, ctabs, surv);
             if (jrc == E_ARG) {
                 set_error("");  // the program does not fit the one-launch kernel: the per-shot plan runs
                 ok = false;
@@ -2197,10 +2192,10 @@ ps_status ps_circuit_compile(ps_state *h, const ps_op *ops_in, uint64_t nops, co
                 FrameRangeDev *dr = nullptr;
                 FrameSlotDev *dsl = nullptr;
                 FrameChanTab *dct = nullptr;
-                uint32_t *dsv = nullptr, *ds64 = nullptr, *dev = nullptr;
+                uint32_t *dsv = nullptr, *ds64 = nullptr;
                 int32_t *dnvr = nullptr;
                 if (upload(h, c->owned, ranges, &dr) || upload(h, c->owned, fslots, &dsl) ||
-                    upload(h, c->owned, fs64, &ds64) || upload(h, c->owned, fev, &dev) || upload(h, c->owned, ctabs, &dct) ||
+                    upload(h, c->owned, fs64, &ds64) || upload(h, c->owned, ctabs, &dct) ||
                     upload(h, c->owned, surv, &dsv) || upload(h, c->owned, nvr, &dnvr))
                     return bail(E_CUDA);
                 job.nv_range = dnvr;
@@ -2214,7 +2209,6 @@ ps_status ps_circuit_compile(ps_state *h, const ps_op *ops_in, uint64_t nops, co
                 job.ranges = dr;
                 job.slot = dsl;
                 job.slot_s64 = ds64;
-                job.slot_event = dev;
                 {  // the error word (offset 0) and the broadcast's counters (offsets 16, 24)
                     void *pe = nullptr;
                     if (dev_alloc(h, &pe, 32) != OK) return bail(E_NOMEM);

@@ -728,4 +728,42 @@ void FrameBuilder::linearize(uint32_t max_rows) {
     op_tab_end_.clear();
 }
 
+void FrameProgram::pack_noise() {
+    nrows.clear();
+    slot_rows.assign(slot_off.size(), SlotRows{});
+    std::vector<uint32_t> bases;  // first slot of each sampled segment, in order
+    for (const Launch &L : launches)
+        if (L.seg >= 0) bases.push_back((uint32_t)ops[L.op0].arg);
+    bases.push_back((uint32_t)slot_off.size());
+    for (size_t k = 0; k + 1 < bases.size(); ++k)
+        for (uint32_t q = bases[k]; q + 1 < bases[k + 1]; ++q) {
+            SlotRows &r = slot_rows[q];
+            r.t0 = (uint32_t)nrows.size();
+            for (uint32_t c = 0; c < 4; ++c) {
+                std::vector<uint16_t> rows;
+                for (uint32_t t = slot_off[q]; t < slot_off[q + 1]; ++t)
+                    if ((tab[t] >> (28 + c)) & 1u) rows.push_back((uint16_t)(tab[t] & kFrameRowMask));
+                r.len[c] = (uint16_t)rows.size();
+                if (rows.size() <= kSlotShort) {
+                    std::copy(rows.begin(), rows.end(), r.rows[c]);
+                    continue;
+                }
+                if (rows.size() & 1) rows.push_back(0);
+                nrows.insert(nrows.end(), rows.begin(), rows.end());
+            }
+        }
+    std::vector<uint32_t> kept;
+    for (Launch &L : launches) {
+        const uint32_t at = (uint32_t)kept.size(), shift = at - L.tab0;
+        kept.insert(kept.end(), tab.begin() + L.tab0, tab.begin() + L.tab1);
+        for (uint32_t i = L.op0; i < L.op1; ++i)
+            if ((ops[i].kind & 0xFFu) != F_NOISE) ops[i].off += shift;
+        L.tab1 = (uint32_t)kept.size();
+        L.tab0 = at;
+        kept.resize((kept.size() + 3) & ~(size_t)3, 0u);
+    }
+    tab.swap(kept);
+    slot_off.clear();
+}
+
 }  // namespace ps

@@ -60,19 +60,24 @@ __device__ __forceinline__ int job_of(const int64_t *__restrict__ first, int njo
 // One CTA of NW warps per (range with channels, shot-word) of a job: the
 // XOR its channel outcomes make on the signs of the word's 64 shots.  A
 // first pass draws every channel's first number (a Philox block gives the
-// first numbers of four consecutive channel events: lane t draws the block
-// of group t, and in slice q lane t takes event 32q + t, whose number it
-// gets by shuffle, so that the S_64 words are read contiguously; no shot of
-// the word is hit unless the number is at least S_64, 94 % of channels at
+// first numbers of four consecutive channel events; no shot of the word is
+// hit unless the number is at least S_64, 94 % of channels at
 // p = 1e-3) and lists the hit channels with their first numbers.  Then a
-// thread per hit samples its word (channel_word_est_hit: the same draws as
-// every other form) and flips its slot's rows in the sum (32-bit shared
-// atomics: XORs commute, and two slots may share a row).  MASKS: a slot's
-// rows are four bit masks over the rows (J.smask, written by the walk of
-// ps_walk.h) instead of a list; off: not 0 on the device when the launch has
-// nothing to do.
+// lane per hit samples its word (channel_word_est_hit: the same draws as
+// every other form) and the rows of what it found are flipped in the sum
+// (32-bit shared atomics: XORs commute, and two slots may share a row).
+// MASKS: a slot's rows are bit masks over the rows (J.smask, written by the
+// walk of ps_walk.h) instead of lists; off: not 0 on the device when the
+// launch has nothing to do.
+// Bound by instructions alone (the samplers' divergent loops) and by the
+// latency of its loads beside the broadcast, so loads are few and early.  At d
+// = 21, p = 5e-3, 50,001 shots: 1.10 ms alone, 2.12 beside the broadcast; with
+// a Philox block per channel, its rows as one list for all four components
+// found by binary search, tables behind generic pointers and S_64 words and
+// records loaded where they are needed it took 1.79 and 3.2.  At d = 15, p =
+// 1e-3, 16,384 shots: 0.065 and 0.085, before 0.090 and 0.176.
 template <int NW, bool MASKS>
-__global__ void __launch_bounds__(32 * NW) noise_vec_kernel(const FrameJobDev *__restrict__ jobs, int njobs,
+__global__ void __launch_bounds__(32 * NW, 32 / NW) noise_vec_kernel(const FrameJobDev *__restrict__ jobs, int njobs,
                                                             const int64_t *__restrict__ ncta0,
                                                             const int32_t *__restrict__ off) {
     extern __shared__ __align__(16) u64 sm[];
@@ -90,26 +95,16 @@ __global__ void __launch_bounds__(32 * NW) noise_vec_kernel(const FrameJobDev *_
     u64 *const acc = sm;
     uint32_t *const shit = reinterpret_cast<uint32_t *>(sb8 + SL.hit);  // hit channels: count, then (channel, first draw)
     uint32_t *const shitl = shit + 2;
-    u64 *const shm = reinterpret_cast<u64 *>(sb8 + SL.hm);               // the chunk's outcome masks (4 a hit)
-    uint32_t *const sht0 = reinterpret_cast<uint32_t *>(sb8 + SL.ht0);   // first row entry of each
-    uint32_t *const shlen = reinterpret_cast<uint32_t *>(sb8 + SL.hlen); // its row count
-    uint32_t *const shpre = reinterpret_cast<uint32_t *>(sb8 + SL.hpre); // prefix of the counts
-    uint32_t *const swsum = reinterpret_cast<uint32_t *>(sb8 + SL.wsum); // per-warp sums
-    const uint32_t *const gtab = J.tab;
+    u64 *const qf = reinterpret_cast<u64 *>(sb8 + SL.qf) + 128 * wid;        // this warp's queue: shots ...
+    uint2 *const qd = reinterpret_cast<uint2 *>(sb8 + SL.qd) + 128 * wid;    // ... first row entry and count
     const RunParams rp = *J.rp;
-    const FrameChanTab *ctab = J.ctab;
-    const uint64_t *thr = J.thr;
-    const uint32_t *surv = J.surv;
+    FrameChanTab *const sctab = reinterpret_cast<FrameChanTab *>(sb8 + SL.tabs);
+    uint64_t *const sthr = reinterpret_cast<uint64_t *>(sctab + J.n_ctab);
+    uint32_t *const ssurv = reinterpret_cast<uint32_t *>(sthr + J.n_thr);
     if (J.stage_tabs) {
-        FrameChanTab *c2 = reinterpret_cast<FrameChanTab *>(sb8 + SL.tabs);
-        uint64_t *t2 = reinterpret_cast<uint64_t *>(c2 + J.n_ctab);
-        uint32_t *s2 = reinterpret_cast<uint32_t *>(t2 + J.n_thr);
-        for (uint32_t i = tid; i < J.n_ctab; i += NT) c2[i] = J.ctab[i];
-        for (uint32_t i = tid; i < J.n_thr; i += NT) t2[i] = J.thr[i];
-        for (uint32_t i = tid; i < J.n_surv; i += NT) s2[i] = J.surv[i];
-        ctab = c2;
-        thr = t2;
-        surv = s2;
+        for (uint32_t i = tid; i < J.n_ctab; i += NT) sctab[i] = J.ctab[i];
+        for (uint32_t i = tid; i < J.n_thr; i += NT) sthr[i] = J.thr[i];
+        for (uint32_t i = tid; i < J.n_surv; i += NT) ssurv[i] = J.surv[i];
     }
     for (int64_t i = tid; i < Wp; i += NT) acc[i] = 0ull;
     if (tid == 0) *shit = 0u;
@@ -128,135 +123,139 @@ __global__ void __launch_bounds__(32 * NW) noise_vec_kernel(const FrameJobDev *_
             shitl[2 * at + 1] = u;
         }
     };
-    if (L.ev0 >= 0) {
+    {
         const uint64_t e0 = rp.event_base + (uint64_t)L.ev0, g0 = e0 >> 2;
         const int64_t ngroups = (int64_t)(((e0 + (uint64_t)L.nslots - 1) >> 2) - g0 + 1);
-        for (int64_t wb = 32 * (int64_t)wid; wb < ngroups; wb += 32 * NW) {  // the warp's 32 groups
-            u32x4 blk{};
-            if (wb + lane < ngroups)
-                blk = draw_block(rp.seed, g0 + (uint64_t)(wb + lane), rp.word_base + (uint64_t)k, 0u, TAG_NOISE_FIRST);
+        // A lane takes a block's four events.  Their S_64 words are fetched a
+        // turn ahead: beside the broadcast a load takes microseconds.
+        const int32_t off0 = (int32_t)(4 * g0 - e0);  // event c of group g is slot 4 g + c + off0
+        uint32_t lim[4];
+        auto fetch = [&](int32_t g) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int src = 8 * q + (lane >> 2);
-                uint32_t x[4];
+            for (int c = 0; c < 4; ++c) {
+                const int32_t sl = 4 * g + c + off0;
+                lim[c] = sl >= 0 && sl < L.nslots ? __ldg(s64 + sl) : 0xFFFFFFFFu;
+            }
+        };
+        fetch(tid);
+        for (int32_t gb = 32 * wid; gb < (int32_t)ngroups; gb += NT) {
+            const int32_t g = gb + lane;
+            uint32_t now[4];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) x[c] = __shfl_sync(0xffffffffu, blk.v[c], src);
-                const uint32_t u = (lane & 3) == 0 ? x[0] : (lane & 3) == 1 ? x[1] : (lane & 3) == 2 ? x[2] : x[3];
-                const int64_t sl = (int64_t)(4 * (g0 + (uint64_t)wb)) + 32 * q + lane - (int64_t)e0;
-                const bool hit = sl >= 0 && sl < L.nslots && u >= __ldg(s64 + sl);
-                append(hit, (uint32_t)sl, u);
+            for (int c = 0; c < 4; ++c) now[c] = lim[c];
+            fetch(g + NT);
+            const u32x4 blk =
+                draw_block(rp.seed, g0 + (uint64_t)g, rp.word_base + (uint64_t)k, 0u, TAG_NOISE_FIRST);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int32_t sl = 4 * g + c + off0;
+                append(sl >= 0 && sl < L.nslots && blk.v[c] >= now[c], (uint32_t)sl, blk.v[c]);
             }
-        }
-    } else {
-        for (int64_t ub = 0; ub < L.nslots; ub += NT) {
-            const int64_t unit = ub + tid;
-            bool hit = false;
-            uint32_t u = 0u;
-            if (unit < L.nslots) {
-                u = channel_first_draw(rp.seed, rp.event_base + J.slot_event[L.slot_base + unit], rp.word_base + (uint64_t)k);
-                hit = u >= __ldg(s64 + unit);
-            }
-            append(hit, (uint32_t)unit, u);
         }
     }
     __syncthreads();
-    // The hits, NT at a time: a thread per hit (spread over the warps: hit
-    // c0 + l on lane l / NW of warp l % NW) samples its word, then all
-    // threads apply the chunk's rows together, row entry e on thread e % NT
-    // (its hit by binary search in the prefix of the row counts), so that a
-    // long row list does not hold its warp back.
+    // The hits, 32 at a time per warp: a lane per hit samples its word and
+    // flips the rows of each component it found (X or Z on a or b, one or two
+    // for most hits) that are in the channel's record.  Components with more
+    // rows queue up; then GL lanes take one each, UI of them in flight.  No
+    // barrier between the warps.
+    constexpr int GL = MASKS ? 16 : 32, NG = 32 / GL, UI = 4;
+    const int gl = lane & (GL - 1), grp = lane / GL;
     const uint32_t nhit = *shit;
-    for (uint32_t c0 = 0; c0 < nhit; c0 += NT) {
-        const uint32_t l = (uint32_t)lane * NW + (uint32_t)wid, h = c0 + l;
-        uint32_t len = 0u;
+    auto flip = [&](uint32_t row, u64 f) {
+        unsigned *const rw = reinterpret_cast<unsigned *>(&acc[row]);
+        if ((uint32_t)f) atomicXor(rw, (uint32_t)f);
+        if (f >> 32) atomicXor(rw + 1, (uint32_t)(f >> 32));
+    };
+    FrameSlotDev dn{};  // the next turn's record, on its way
+    auto fetch_rec = [&](uint32_t h) {
+        if (h < nhit) dn = rec[shitl[2 * h]];
+    };
+    const uint32_t h0 = (uint32_t)lane * NW + (uint32_t)wid;  // spread over the warps
+    fetch_rec(h0);
+    for (uint32_t c0 = 0; c0 + (uint32_t)wid < nhit; c0 += NT) {
+        const uint32_t h = c0 + h0;
+        ChannelWord m{0ull, 0ull, 0ull, 0ull};
+        const FrameSlotDev d = dn;
+        fetch_rec(h + NT);
         if (h < nhit) {
             const uint32_t s0 = shitl[2 * h];
-            const FrameSlotDev d = rec[s0];
-            const uint32_t tb = d.lt & 0xFFFu;
-            ChannelWord m{0ull, 0ull, 0ull, 0ull};
-            if (tb != kFrameNoHit) {  // (a channel that never hits has S_64 = 2^32 - 1)
-                const FrameChanTab ct = ctab[tb];
-                const uint32_t ev = L.ev0 >= 0 ? (uint32_t)L.ev0 + s0 : J.slot_event[L.slot_base + s0];
-                m = channel_word_est_hit(rp.seed, rp.event_base + ev, rp.word_base + (uint64_t)k, shitl[2 * h + 1],
-                                         thr + ct.thr_off, ct.count, surv + ct.surv_off, ct.est);
-                len = d.lt >> 12;
-            }
-            shm[4 * l + 0] = m.fxa;
-            shm[4 * l + 1] = m.fza;
-            shm[4 * l + 2] = m.fxb;
-            shm[4 * l + 3] = m.fzb;
-            sht0[l] = d.t0;
-            if (MASKS) len = (m.fxa | m.fza | m.fxb | m.fzb) != 0ull;
-        }
-        shlen[l] = len;
-        __syncthreads();
-        if (MASKS) {
-            // (hit, word of the row masks) pairs over the threads; a mask is
-            // read only where the hit has that Pauli
-            const uint32_t ww = (uint32_t)J.ww;
-            for (uint32_t e = tid; e < (uint32_t)NT * ww; e += NT) {
-                const uint32_t lo = e / ww, t = e - lo * ww;
-                if (!shlen[lo]) continue;
-                const u64 fxa = shm[4 * lo + 0], fza = shm[4 * lo + 1], fxb = shm[4 * lo + 2], fzb = shm[4 * lo + 3];
-                const u64 *const mk = J.smask + (size_t)sht0[lo] * 4 * ww + t;
-                const u64 m0 = fxa ? mk[0] : 0ull, m1 = fza ? mk[ww] : 0ull;
-                const u64 m2 = fxb ? mk[2 * ww] : 0ull, m3 = fzb ? mk[3 * ww] : 0ull;
-                for (u64 v = m0 | m1 | m2 | m3; v; v &= v - 1) {
-                    const int b = __ffsll((long long)v) - 1;
-                    u64 f = 0ull;
-                    if ((m0 >> b) & 1ull) f ^= fxa;
-                    if ((m1 >> b) & 1ull) f ^= fza;
-                    if ((m2 >> b) & 1ull) f ^= fxb;
-                    if ((m3 >> b) & 1ull) f ^= fzb;
-                    unsigned *rw = reinterpret_cast<unsigned *>(&acc[64 * t + b]);
-                    if ((uint32_t)f) atomicXor(rw, (uint32_t)f);
-                    if (f >> 32) atomicXor(rw + 1, (uint32_t)(f >> 32));
+            if (d.table != kFrameNoHit) {  // (a channel that never hits has S_64 = 2^32 - 1)
+                const uint64_t ev = rp.event_base + L.ev0 + s0, word = rp.word_base + (uint64_t)k;
+                if (J.stage_tabs) {  // (a branch, so that the compiler knows the tables for shared memory)
+                    const FrameChanTab ct = sctab[d.table];
+                    m = channel_word_est_hit(rp.seed, ev, word, shitl[2 * h + 1], sthr + ct.thr_off, ct.count,
+                                             ssurv + ct.surv_off, ct.est);
+                } else {
+                    const FrameChanTab ct = J.ctab[d.table];
+                    m = channel_word_est_hit(rp.seed, ev, word, shitl[2 * h + 1], J.thr + ct.thr_off, ct.count,
+                                             J.surv + ct.surv_off, ct.est);
                 }
             }
-            __syncthreads();  // the chunk applied before the next one reuses its arrays
-            continue;
         }
-        // exclusive prefix of the row counts, in chunk order (thread tid
-        // takes entry tid here)
-        const uint32_t mine = shlen[tid];
-        uint32_t x = mine;
+        const u64 f4[4] = {m.fxa, m.fza, m.fxb, m.fzb};
+        uint32_t mine = 0u;  // components for the queue
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const bool on = f4[c] != 0ull;
+            if (!MASKS)
+#pragma unroll
+                for (uint32_t r = 0; r < FrameProgram::kSlotShort; ++r)
+                    if (on && r < d.len[c] && d.len[c] <= FrameProgram::kSlotShort) flip(d.rows[c][r], f4[c]);
+            mine += on && (MASKS || d.len[c] > FrameProgram::kSlotShort);
+        }
+        if (!__any_sync(0xffffffffu, mine != 0u)) continue;
+        uint32_t at = mine;  // inclusive prefix over the warp
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
+            const uint32_t y = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= o) at += y;
         }
-        if (lane == 31) swsum[wid] = x;
-        __syncthreads();
-        uint32_t woff = 0u, total = 0u;
+        const uint32_t total = __shfl_sync(0xffffffffu, at, 31);
+        at -= mine;
+        uint32_t t0 = d.t0;
 #pragma unroll
-        for (int q = 0; q < NW; ++q) {
-            const uint32_t vq = swsum[q];
-            woff += q < wid ? vq : 0u;
-            total += vq;
-        }
-        shpre[tid] = woff + x - mine;
-        __syncthreads();
-        for (uint32_t e = tid; e < total; e += NT) {
-            // the last hit with shpre <= e: it has rows (one without any
-            // shares its prefix with the next, and the last one's prefix is
-            // the total)
-            uint32_t lo = 0u, hi = NT - 1u;
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi + 1u) >> 1;
-                if (shpre[mid] <= e) lo = mid;
-                else hi = mid - 1u;
+        for (int c = 0; c < 4; ++c) {
+            const bool lng = d.len[c] > FrameProgram::kSlotShort;
+            if (f4[c] && (MASKS || lng)) {
+                qf[at] = f4[c];
+                qd[at] = MASKS ? make_uint2(4u * d.t0 + (uint32_t)c, 0u) : make_uint2(t0, d.len[c]);
+                ++at;
             }
-            const uint32_t vr = __ldg(gtab + sht0[lo] + (e - shpre[lo])), sel = vr >> 28;
-            u64 f = 0ull;  // row | sel << 28: X on rows with z, Z on rows with x
-            if (sel & 1u) f ^= shm[4 * lo + 0];
-            if (sel & 2u) f ^= shm[4 * lo + 1];
-            if (sel & 4u) f ^= shm[4 * lo + 2];
-            if (sel & 8u) f ^= shm[4 * lo + 3];
-            unsigned *rw = reinterpret_cast<unsigned *>(&acc[vr & kFrameRowMask]);
-            if ((uint32_t)f) atomicXor(rw, (uint32_t)f);
-            if (f >> 32) atomicXor(rw + 1, (uint32_t)(f >> 32));
+            if (lng) t0 += (d.len[c] + 1u) & ~1u;
         }
-        __syncthreads();  // the chunk applied before the next one reuses its arrays
+        __syncwarp();
+        for (uint32_t i0 = (uint32_t)grp; i0 < total; i0 += NG * UI) {
+            u64 f[UI];
+            uint2 e[UI];
+            u64 v[UI];  // the row mask's word, or two rows
+#pragma unroll
+            for (int u = 0; u < UI; ++u) {
+                const uint32_t i = i0 + NG * u;
+                const bool on = i < total;
+                f[u] = on ? qf[i] : 0ull;
+                e[u] = on ? qd[i] : make_uint2(0u, 0u);
+                if (MASKS)
+                    v[u] = on && gl < J.ww ? J.smask[(size_t)e[u].x * J.ww + gl] : 0ull;
+                else
+                    v[u] = 2u * gl < e[u].y ? *reinterpret_cast<const uint32_t *>(J.nrows + e[u].x + 2 * gl) : 0u;
+            }
+#pragma unroll
+            for (int u = 0; u < UI; ++u) {
+                if (MASKS) {
+                    for (u64 x = v[u]; x; x &= x - 1) flip(64 * gl + __ffsll((long long)x) - 1, f[u]);
+                } else {
+                    if (2u * gl < e[u].y) flip((uint32_t)v[u] & 0xFFFFu, f[u]);
+                    if (2u * gl + 1 < e[u].y) flip((uint32_t)v[u] >> 16, f[u]);
+                    for (uint32_t r = 2u * (GL + gl); r < e[u].y; r += 2u * GL) {  // more than 64 rows
+                        const uint32_t rr = *reinterpret_cast<const uint32_t *>(J.nrows + e[u].x + r);
+                        flip(rr & 0xFFFFu, f[u]);
+                        if (r + 1 < e[u].y) flip(rr >> 16, f[u]);
+                    }
+                }
+            }
+        }
+        __syncwarp();  // the queue applied before it is filled again
     }
     __syncthreads();
     u64 *const out = J.nvec + ((int64_t)v * w + k) * Wp;

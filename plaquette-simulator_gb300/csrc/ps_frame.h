@@ -106,6 +106,25 @@ struct FrameProgram {
     // outcomes depend on no sign, so a launch draws them all up front.
     std::vector<int32_t> rand_meas;
     std::vector<Launch> launches;
+    // The channels' rows as the device reads them (pack_noise): per slot of
+    // slot_off, for each component fx(a), fz(a), fx(b), fz(b) the rows it
+    // flips.  Most are a few (at d = 21, 85 % of the lists hold at most four
+    // rows, and 10 % hold three quarters of all rows): up to kSlotShort are
+    // in the slot itself, longer lists follow one another from nrows[t0],
+    // each from an even index.  A hit has few of the components, and reads
+    // only their rows.
+    static constexpr uint32_t kSlotShort = 4;
+    struct SlotRows {
+        uint32_t t0;
+        uint16_t len[4];
+        uint16_t rows[4][kSlotShort];
+    };
+    std::vector<uint16_t> nrows;
+    std::vector<SlotRows> slot_rows;
+    // Builds them and takes the channels' entries out of tab (after
+    // FrameBuilder::finish and linearize): what is left of tab is each
+    // launch's measurement range, from a multiple of 4.
+    void pack_noise();
 };
 
 // Host-side simulation of the shared x / z bits and emission of the sign

@@ -10,18 +10,17 @@
 
 namespace ps {
 
-// A channel of a sign program, indexed like slot_off (slot_base + slot):
-// its rows tab[t0, t0 + len) and its table, packed as lt = len << 12 |
-// table; table kFrameNoHit marks a channel that never hits (total
-// probability 0).  Its S_64 word (a first draw below it hits no shot of the
-// word) and its event offset are kept in arrays of their own.
-struct FrameSlotDev {
-    uint32_t t0;
-    uint32_t lt;
+// A channel of a sign program, in the order of its range's events: its row
+// lists (FrameProgram::SlotRows) and its table; table kFrameNoHit marks
+// a channel that never hits (total probability 0).  Its S_64 word (a first
+// draw below it hits no shot of the word) is kept in an array of its own.
+struct __align__(16) FrameSlotDev {
+    uint32_t t0, table;
+    uint16_t len[4];
+    uint16_t rows[4][FrameProgram::kSlotShort];
 };
 constexpr uint32_t kFrameNoHit = 4095;
 constexpr uint32_t kFrameMaxTables = 4095;
-constexpr uint32_t kFrameMaxSlotRows = (1u << 20) - 1;
 
 // A distinct channel table: thresholds at thr + thr_off (count + 1 entries),
 // survival products at surv + surv_off (channel_surv_table) and the factors
@@ -43,16 +42,14 @@ constexpr uint32_t kFrameTabStage = 4096;
 // channel outcomes, drawn and applied first, then ops [op0, op1).
 struct FrameRangeDev {
     int32_t nslots;          // the segment's channels (0: none)
-    uint32_t slot_base;      // slot_off index of the segment's first slot
     uint32_t op0, op1;
     uint32_t tab0a, ntab16;  // staged tab words: 16-byte chunks from tab0a (stage = 1)
     uint32_t rand0, nrand;   // rand_meas[rand0, rand0 + nrand): the range's random measurements
     uint32_t stage;          // 1: ops and tab range staged in shared memory
-    int32_t ev0;             // >= 0: the channels' events are ev0, ev0 + 1, ... (first draws by groups of four)
+    uint32_t ev0;            // the channels' events are ev0, ev0 + 1, ...
     uint32_t s64_base;       // slot_s64 index of the segment's first S_64 word (a multiple of 4)
-    uint32_t rec_base;       // slot index of the segment's first channel record (even: 16-byte aligned)
+    uint32_t rec_base;       // slot index of the segment's first channel record
     int32_t nv;              // >= 0: its noise vectors are block nv of the job's nvec
-    uint32_t pad;
 };
 
 // One job: a sign program over the signs R of every shot-word of one state.
@@ -72,8 +69,8 @@ struct FrameJobDev {
     int64_t nm;
     const uint64_t *thr;  // channel threshold tables
     const FrameSlotDev *slot;    // channel records, per range from rec_base
+    const uint16_t *nrows;       // their longer row lists
     const uint32_t *slot_s64;    // S_64 of every channel (0xFFFFFFFF for one that never hits), per range from s64_base
-    const uint32_t *slot_event;  // event offset of every channel, like slot (ranges with ev0 < 0 read it)
     const FrameChanTab *ctab;
     const uint32_t *surv;
     const RunParams *rp;
@@ -129,29 +126,25 @@ __host__ __device__ inline FrameSmem frame_smem_layout(const FrameJobDev &j) {
 // Shared memory the sign kernel needs for a job.
 inline size_t frame_job_smem(const FrameJobDev &j) { return frame_smem_layout(j).total; }
 
-// The noise kernel runs kNoiseWarps warps a CTA and takes the hits of its
-// range kNoiseChunk (one per thread) at a time.
+// The noise kernel runs kNoiseWarps warps a CTA; each takes 32 hits of its
+// range at a time.
 constexpr int kNoiseWarps = 4;
-constexpr uint32_t kNoiseChunk = 32 * kNoiseWarps;
 // The noise kernel asks for at least this much shared memory a CTA, which
 // keeps it to six CTAs an SM.
 constexpr size_t kNoiseSmemFloor = 36 * 1024;
 
 // Shared-memory layout of the noise kernel for one job: the noise vector
-// being summed (Wp words), a chunk of hits (outcome masks, first row entry,
-// row count, prefix of the counts), per-warp sums, the channel tables when
-// staged, the hit list (count, then channel and first draw of each hit).
+// being summed (Wp words), each warp's queue of hit components (their shots
+// [128], then rows and counts [128]), the channel tables when staged, the hit
+// list (count, then channel and first draw of each hit).
 struct NoiseSmem {
-    size_t hm, ht0, hlen, hpre, wsum, tabs, hit, total;
+    size_t qf, qd, tabs, hit, total;
 };
 __host__ __device__ inline NoiseSmem noise_smem_layout(const FrameJobDev &j) {
     NoiseSmem L;
-    L.hm = (size_t)frame_wp(j.n) * 8;
-    L.ht0 = L.hm + (size_t)kNoiseChunk * 32;
-    L.hlen = L.ht0 + (size_t)kNoiseChunk * 4;
-    L.hpre = L.hlen + (size_t)kNoiseChunk * 4;
-    L.wsum = L.hpre + (size_t)kNoiseChunk * 4;
-    L.tabs = L.wsum + 16 * 4;
+    L.qf = (size_t)frame_wp(j.n) * 8;
+    L.qd = L.qf + (size_t)kNoiseWarps * 128 * 8;
+    L.tabs = L.qd + (size_t)kNoiseWarps * 128 * 8;
     L.hit = frame_align16(L.tabs + (j.stage_tabs ? (size_t)j.n_ctab * sizeof(FrameChanTab) + (size_t)j.n_thr * 8 +
                                                        (size_t)j.n_surv * 4
                                                  : 0));

@@ -203,8 +203,10 @@ int launch_segment(cudaStream_t stream, u64 *X, u64 *Z, u64 *R, int64_t n, int64
 // ps_frame.cu (shared-x/z runs; the launches are declared in ps_frame_dev.h)
 size_t frame_smem_bytes(int64_t n);
 // Staging buffers of a sign program's ranges stay within this (beside the
-// signs); ranges that need more read their ops from global memory.
-constexpr size_t kFrameStageMax = 100 * 1024;
+// signs); ranges that need more read their ops from global memory.  At d = 21
+// that keeps two CTAs on an SM, where the two ranges with random measurements
+// would leave room for one (0.51 ms, with 100 KB 0.67).
+constexpr size_t kFrameStageMax = 48 * 1024;
 
 // ps_gates.cu (compiled-circuit form of the per-op kernels)
 // The channel of a compiled plain run in one launch (sampling and sign
