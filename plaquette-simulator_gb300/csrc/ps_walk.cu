@@ -102,15 +102,25 @@ __global__ void __launch_bounds__(256) walk_gather_kernel(const u64 *__restrict_
 
 // --------------------------------------------------------------- walk
 constexpr int kWalkThreads = 512;
+constexpr int kWalkShares = 16;  // CTAs, each with a share of the outputs
 constexpr int kWalkWarps = kWalkThreads / 32;
+constexpr int kPivotFlip = 1 << 16;  // the pivot row's constant
 
 // Row strides in words: odd, so that the words of consecutive columns (or
 // rows) that a warp reads fall on distinct bank pairs.
 __host__ __device__ inline int walk_wp(int ww) { return ww | 1; }
 __host__ __device__ inline int walk_np(int nw) { return nw | 1; }
 
+// A random measurement's columns over the warps: column j is lane j / 16 of
+// warp (j / 16 + j) % 16.  Neighbouring qubits fall on different warps (the
+// pivot row's Paulis are often on neighbours), and a warp's columns on
+// distinct bank pairs.
+static_assert(kWalkWarps == 16 && kWalkMaxQubits <= 32 * kWalkWarps, "one column a thread");
+__device__ __forceinline__ int walk_col(int warp, int k) { return 16 * k + ((warp - k) & 15); }
+__device__ __forceinline__ int walk_owner(int j) { return ((j >> 4) + j) & 15; }
+
 struct WalkSmem {
-    size_t zc, f, stab, part, list, total;
+    size_t zc, f, stab, part, total;
 };
 __host__ __device__ inline WalkSmem walk_layout(int64_t n) {
     const int ww = (int)((2 * n + 1 + 63) / 64), nw = (int)((n + 63) / 64);
@@ -120,27 +130,35 @@ __host__ __device__ inline WalkSmem walk_layout(int64_t n) {
     L.f = 2 * col;
     L.stab = L.f + 16 * 8;
     L.part = (L.stab + st + 15) & ~(size_t)15;
-    L.list = L.part + (size_t)kWalkWarps * 16 * 16;
-    L.total = L.list + (size_t)n * 4;
+    L.total = L.part + 2 * (size_t)kWalkWarps * 16 * 16;
     return L;
 }
 
-// One CTA follows one tableau through the circuit.  Its columns are bit
+// A CTA follows one tableau through the circuit.  Its columns are bit
 // vectors over the rows, so a gate is a few words' XOR for all rows: half a
 // warp takes a gate, a lane per word, so that a column is one conflict-free
 // shared-memory access (lanes over gates instead measured 1.9x slower: 4-way
 // bank conflicts on the columns).  Nothing here scales with the shots: the
-// time is the warps' shared-memory accesses and instructions on one SM and
-// the latency of the steps (13 rounds at d = 13, 4,368 measurements: 0.33 ms,
-// about 1 us for a layer's gates, 1.2 us for its channels, 19 us for a phase
-// of 336 deterministic measurements; a random measurement on 450 qubits 1.4
-// us).
+// time is the warps' instructions and shared-memory accesses on one SM and
+// the latency of the steps.
+//
+// What has to be followed is little beside what has to be worked out from
+// it for the signs (channels' rows, deterministic outcomes, the constants
+// and lists of random ones), and nothing of the latter is read again.  So
+// kWalkShares CTAs follow the same tableau, without a word between them,
+// and each writes its share of the outputs.  13 rounds at d = 13 (4,368
+// measurements): 0.39 ms in one CTA, 0.31 in 8, 0.27 in 16; 5 qubits and 7
+// measurements are no slower for it (46 us).
 //
 // A measurement phase goes position by position.  If its column has a
-// stabilizer row set, the measurement is random; every warp finds the pivot
-// by itself.  It multiplies the pivot row into every other row with x(q)
-// set, all rows of a word at once (bit-sliced mod-4 phase counters), over
-// the columns where the pivot row has a Pauli: two barriers.  Otherwise the
+// stabilizer row set, the measurement is random: the pivot row is multiplied
+// into every other row with x(q) set, all rows of a word at once (bit-sliced
+// mod-4 phase counters), over the columns where the pivot row has a Pauli.
+// Each warp finds those among its own columns, and the warp that holds the
+// next position's column looks for that one's pivot as soon as it is done,
+// so a random measurement is one barrier (90 distillation blocks, 450
+// qubits: 0.83 us each; with a list of the columns that all warps share and
+// the pivot found by every warp, two barriers and 1.4 us).  Otherwise the
 // run of deterministic measurements from there on is done at once.  A
 // deterministic outcome is the product of the stabilizers that the column's
 // destabilizer rows select, its sign the summed phase of that product;
@@ -148,27 +166,30 @@ __host__ __device__ inline WalkSmem walk_layout(int64_t n) {
 // row-major copy of the stabilizers that is made again after x / z changed.
 __global__ void __launch_bounds__(kWalkThreads, 1) walk_kernel(WalkDev d, int reset, cudaGraphConditionalHandle fall) {
     extern __shared__ __align__(16) u64 sm[];
-    __shared__ int s_first[2], s_cnt[2];
+    __shared__ int s_first[2];
+    // the next position's pivot (-1: deterministic) and the rows a random one multiplies
+    __shared__ int s_pivot[2];
+    __shared__ u64 s_rows[2][16];
     __shared__ int32_t s_mq[kWalkThreads];
     if (!reset && *d.bad) {  // the per-shot kernels' turn (a conditional part of the graph)
-        if (fall && threadIdx.x == 0) cudaGraphSetConditional(fall, 1u);
+        if (fall && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(fall, 1u);
         return;
     }
+    const int share = blockIdx.x, shares = gridDim.x;  // which of the outputs this CTA writes
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = d.n, W = 2 * n + 1, ww = d.ww, nw = d.nw, wp = walk_wp(ww), np = walk_np(nw);
     const WalkSmem SL = walk_layout(n);
     char *const b8 = reinterpret_cast<char *>(sm);
     u64 *const xc = sm, *const zc = reinterpret_cast<u64 *>(b8 + SL.zc);
+    uint32_t *const xc32 = reinterpret_cast<uint32_t *>(xc), *const zc32 = reinterpret_cast<uint32_t *>(zc);
     u64 *const F = reinterpret_cast<u64 *>(b8 + SL.f);
     u64 *const sx = reinterpret_cast<u64 *>(b8 + SL.stab), *const sz = sx + (size_t)n * np;
-    ulonglong2 *const part = reinterpret_cast<ulonglong2 *>(b8 + SL.part);  // a random one's phases: [warp][word]
-    uint32_t *const list = reinterpret_cast<uint32_t *>(b8 + SL.list);
+    ulonglong2 *const part = reinterpret_cast<ulonglong2 *>(b8 + SL.part);  // a random one's phases: [2][warp][word]
 
     for (int i = tid; i < n * wp; i += kWalkThreads) xc[i] = zc[i] = 0ull;
     if (tid < 16) F[tid] = 0ull;
     if (tid < 2) {
         s_first[tid] = 0x7FFFFFFF;
-        s_cnt[tid] = 0;
     }
     __syncthreads();
     if (reset) {  // |0...0>: x(i, i), z(i + n, i) and the scratch row's sign
@@ -195,26 +216,31 @@ __global__ void __launch_bounds__(kWalkThreads, 1) walk_kernel(WalkDev d, int re
     const u64 rm_stab = row_mask(lane, n, 2 * n), rm_destab = row_mask(lane, 0, n), rm_rows = row_mask(lane, 0, 2 * n);
     // A step's ops as the threads hold them, fetched a step ahead (an op's
     // load is several steps' work away): half-warp hw does ops hw, hw + HW,
-    // ..., and its lane t holds the one of round t.  Channels and sign ops
-    // past 16 rounds are read when due.
+    // ..., and its lane t holds the one of round t (channels: of this CTA's
+    // share).  Ops past 16 rounds are read when due.
     constexpr int HW = kWalkThreads / 16;
-    const int t = lane & 15, hw = tid >> 4;
+    const int t = lane & 15, hw = tid >> 4, jw = walk_col(warp, lane);
     const WalkStep none{};
     auto step = [&](int i) { return i < d.nsteps ? d.steps[i] : none; };
+    const int NS = HW * shares;  // channels a round, over all CTAs
     auto held = [&](const uint32_t *ops, int o0, int o1) {
         const int o = o0 + hw + HW * t;
         return o < o1 ? ops[o] : 0u;
     };
+    auto held_slot = [&](int o0, int o1) {
+        const int o = o0 + hw * shares + share + NS * t;
+        return o < o1 ? d.slots[o] : 0u;
+    };
     WalkStep st = step(0), st1 = step(1);
     uint32_t hg = st.phase ? 0u : held(d.gates, st.i0, st.i1), hs = held(d.signs, st.s0, st.s1),
-             hn = held(d.slots, st.n0, st.n1);
+             hn = held_slot(st.n0, st.n1);
     bool dirty = true;  // the row-major stabilizers are stale
     u64 fl = 0ull;      // the segment's constant flips, this thread's share of word t
     int fi = 0, ci = 0;
     for (int si = 0; si < d.nsteps; ++si) {
         const WalkStep st2 = step(si + 2);
         const uint32_t hg1 = st1.phase ? 0u : held(d.gates, st1.i0, st1.i1), hs1 = held(d.signs, st1.s0, st1.s1),
-                       hn1 = held(d.slots, st1.n0, st1.n1);
+                       hn1 = held_slot(st1.n0, st1.n1);
         if (!st.phase) {
             const int ng = st.i1 - st.i0;  // at most 511: disjoint qubits
             for (int r = 0; r * HW < ng; ++r) {
@@ -252,11 +278,11 @@ __global__ void __launch_bounds__(kWalkThreads, 1) walk_kernel(WalkDev d, int re
                 if (code == OP_X) fl ^= z;
                 else if (code == OP_Y) fl ^= x ^ z;
                 else if (code == OP_Z) fl ^= x;
-                else d.rmask[(int64_t)(st.r0 + (int)(o >> 15)) * ww + t] = code == kWalkRecX ? z : x;
+                else if (g % shares == share) d.rmask[(int64_t)(st.r0 + (int)(o >> 15)) * ww + t] = code == kWalkRecX ? z : x;
             }
-            // channels: the rows that their Paulis flip
-            for (int r = 0; st.n0 + r * HW < st.n1; ++r) {
-                const int s = st.n0 + r * HW + hw;
+            // channels: the rows that their Paulis flip, this CTA's share
+            for (int r = 0; st.n0 + r * NS < st.n1; ++r) {
+                const int s = st.n0 + r * NS + hw * shares + share;
                 const uint32_t h = __shfl_sync(kFull, hn, r & 15, 16);
                 if (s >= st.n1 || t >= ww) continue;
                 const uint32_t o = r < 16 ? h : d.slots[s], b = o >> 16;
@@ -277,90 +303,107 @@ __global__ void __launch_bounds__(kWalkThreads, 1) walk_kernel(WalkDev d, int re
         } else {
             dirty = true;
         }
+        // Looks at position m's column, by the warp that holds it: which row is
+        // the pivot, if any, and the rows to multiply.
+        auto publish = [&](int m, int c0) {
+            const int q = s_mq[m - c0] & kWalkQubit;
+            if (warp != walk_owner(q)) return;
+            const u64 col = lane < ww ? xc[q * wp + lane] : 0ull;
+            const unsigned bal = __ballot_sync(kFull, (col & rm_stab) != 0ull);
+            if (!bal) {
+                if (lane == 0) s_pivot[ci] = -1;
+                return;
+            }
+            // random: the lowest stabilizer row with x(q) set is the pivot
+            const int src = __ffs(bal) - 1;
+            const int p = 64 * src + __ffsll((long long)__shfl_sync(kFull, col & rm_stab, src)) - 1 - n;
+            const u64 bp = lane == p >> 6 ? 1ull << (p & 63) : 0ull;
+            const u64 bq = lane == (p + n) >> 6 ? 1ull << ((p + n) & 63) : 0ull;
+            if (lane < 16) s_rows[ci][lane] = col & rm_rows & ~(bp | bq);
+            const u64 f = lane < ww ? F[lane] : 0ull;
+            const bool fp = __any_sync(kFull, (f & bq) != 0ull);
+            if (bp | bq) F[lane] = (f & ~(bp | bq)) | (fp ? bp : 0ull);
+            if (lane == 0) s_pivot[ci] = p | (fp ? kPivotFlip : 0);
+        };
         for (int c0 = st.i0; st.phase && c0 < st.i1; c0 += kWalkThreads) {
             const int c1 = min(st.i1, c0 + kWalkThreads);
             __syncthreads();
             if (c0 + tid < c1) s_mq[tid] = d.mq[c0 + tid];
             __syncthreads();
+            bool known = false;  // the position is published
             for (int pos = c0; pos < c1;) {
-                const int32_t mq = s_mq[pos - c0];
-                const int q = mq & kWalkQubit;
-                const u64 col = lane < ww ? xc[q * wp + lane] : 0ull;
-                const unsigned bal = __ballot_sync(kFull, (col & rm_stab) != 0ull);
-                if (bal) {
-                    // random: the lowest stabilizer row with x(q) set is the pivot
-                    const int src = __ffs(bal) - 1;
-                    const int p = 64 * src + __ffsll((long long)__shfl_sync(kFull, col & rm_stab, src)) - 1 - n;
-                    const int tp = p >> 6, tq = (p + n) >> 6;
-                    const u64 bp = 1ull << (p & 63), bq = 1ull << ((p + n) & 63);
-                    u64 Ml = col & rm_rows;
-                    if (lane == tp) Ml &= ~bp;
-                    if (lane == tq) Ml &= ~bq;
-                    const bool fp = (F[tq] & bq) != 0ull;
-                    const int j = tid;  // (n < 512)
-                    bool xp = false, zp = false;
-                    if (j < n) {
-                        xp = (xc[j * wp + tq] & bq) != 0ull;
-                        zp = (zc[j * wp + tq] & bq) != 0ull;
-                    }
-                    const unsigned lb = __ballot_sync(kFull, xp || zp);
-                    if (lb) {
-                        int base = 0;
-                        if (lane == 0) base = atomicAdd(&s_cnt[ci], __popc(lb));
-                        base = __shfl_sync(kFull, base, 0);
-                        if (xp || zp)
-                            list[base + __popc(lb & ((1u << lane) - 1u))] =
-                                (uint32_t)j | (xp ? 1u << 30 : 0u) | (zp ? 1u << 31 : 0u);
-                    }
+                if (!known) {
+                    publish(pos, c0);
                     __syncthreads();
+                }
+                const int pivot = s_pivot[ci];
+                if (pivot >= 0) {
+                    const int32_t mq = s_mq[pos - c0];
+                    const int q = mq & kWalkQubit;
+                    const bool fp = (pivot & kPivotFlip) != 0;
+                    const int p = pivot & ~kPivotFlip, tp = p >> 6, tq = (p + n) >> 6;
+                    const u64 bp = 1ull << (p & 63), bq = 1ull << ((p + n) & 63);
+                    const u64 M = s_rows[ci][t];
+                    const bool mine = pos % shares == share;
+                    const u64 Ml = mine && lane < 16 ? s_rows[ci][lane] : 0ull;
                     // row p := the pivot row, row p + n := Z_q, the multiplied rows *= the pivot row
-                    if (j < n && !(xp || zp)) {
-                        xc[j * wp + tp] &= ~bp;
-                        zc[j * wp + tp] &= ~bp;
-                    }
-                    if (tid == 0) {
-                        s_cnt[ci ^ 1] = 0;
-                        F[tq] &= ~bq;
-                        F[tp] = (F[tp] & ~bp) | (fp ? bp : 0ull);
-                    }
-                    const int cnt = s_cnt[ci];
-                    const u64 M = __shfl_sync(kFull, Ml, t);
-                    u64 a1 = 0ull, a0 = 0ull;
-                    if (t < ww)
-                        for (int k = tid >> 4; k < cnt; k += kWalkThreads / 16) {
-                            const uint32_t v = list[k];
-                            const int jj = (int)(v & 0xFFFFu), o = jj * wp + t;
-                            const u64 x1 = xc[o], z1 = zc[o];
-                            const u64 x2 = v & (1u << 30) ? ~0ull : 0ull, z2 = v & (1u << 31) ? ~0ull : 0ull;
-                            phase_accumulate(x1, z1, x2, z2, M, a1, a0);
-                            u64 xn = x1 ^ (x2 & M), zn = z1 ^ (z2 & M);
-                            if (t == tp) {
-                                xn = (xn & ~bp) | (x2 & bp);
-                                zn = (zn & ~bp) | (z2 & bp);
-                            }
-                            if (t == tq) {
-                                xn &= ~bq;
-                                zn = (zn & ~bq) | (jj == q ? bq : 0ull);
-                            }
-                            xc[o] = xn;
-                            zc[o] = zn;
+                    bool xp = false, zp = false;
+                    if (jw < n) {
+                        const int op = 2 * jw * wp + (p >> 5), oq = 2 * jw * wp + ((p + n) >> 5);
+                        xp = (xc32[oq] >> ((p + n) & 31)) & 1u;
+                        zp = (zc32[oq] >> ((p + n) & 31)) & 1u;
+                        if (!(xp || zp)) {
+                            xc32[op] &= ~(1u << (p & 31));
+                            zc32[op] &= ~(1u << (p & 31));
                         }
-                    {
+                    }
+                    const unsigned bx = __ballot_sync(kFull, xp), bz = __ballot_sync(kFull, zp);
+                    u64 a1 = 0ull, a0 = 0ull;
+                    for (unsigned todo = bx | bz; todo;) {  // half a warp a column
+                        int k = __ffs(todo) - 1;
+                        todo &= todo - 1;
+                        if (lane >= 16) k = __ffs(todo) - 1;  // (-1: none left)
+                        todo &= todo - 1;
+                        if (k < 0 || t >= ww) continue;
+                        const int jj = walk_col(warp, k), o = jj * wp + t;
+                        const u64 x1 = xc[o], z1 = zc[o];
+                        const u64 x2 = (bx >> k) & 1u ? ~0ull : 0ull, z2 = (bz >> k) & 1u ? ~0ull : 0ull;
+                        if (mine) phase_accumulate(x1, z1, x2, z2, M, a1, a0);
+                        u64 xn = x1 ^ (x2 & M), zn = z1 ^ (z2 & M);
+                        if (t == tp) {
+                            xn = (xn & ~bp) | (x2 & bp);
+                            zn = (zn & ~bp) | (z2 & bp);
+                        }
+                        if (t == tq) {
+                            xn &= ~bq;
+                            zn = (zn & ~bq) | (jj == q ? bq : 0ull);
+                        }
+                        xc[o] = xn;
+                        zc[o] = zn;
+                    }
+                    __syncwarp();
+                    if (mine) {
                         const u64 e1 = __shfl_xor_sync(kFull, a1, 16), e0 = __shfl_xor_sync(kFull, a0, 16);
                         phase_add(a1, a0, e1, e0);
+                        if (lane < 16) part[(ci * kWalkWarps + warp) * 16 + t] = make_ulonglong2(a1, a0);
+                        if (warp == walk_owner(q) && (mq & kWalkReset) && lane < ww)
+                            d.mmask[((int64_t)pos * 2 + 1) * ww + lane] = zc[q * wp + lane];
                     }
-                    if (lane < 16) part[warp * 16 + t] = make_ulonglong2(a1, a0);
+                    ci ^= 1;
+                    known = pos + 1 < c1;
+                    if (known) publish(pos + 1, c0);
                     __syncthreads();
-                    if (warp < ww) {  // warp = word: the warps' partial counters (beside the next position's reads)
-                        const ulonglong2 v = part[(lane & (kWalkWarps - 1)) * 16 + warp];
+                    // a warp per word: the warps' partial counters, the rows and
+                    // constants (beside the next position's reads)
+                    if (mine && warp < ww) {
+                        const ulonglong2 v = part[((ci ^ 1) * kWalkWarps + (lane & (kWalkWarps - 1))) * 16 + warp];
                         u64 b1 = v.x, b0 = v.y;
 #pragma unroll
                         for (int o = kWalkWarps / 2; o > 0; o >>= 1) {
                             const u64 e1 = __shfl_xor_sync(kFull, b1, o), e0 = __shfl_xor_sync(kFull, b0, o);
                             phase_add(b1, b0, e1, e0);
                         }
-                        b1 = __shfl_sync(kFull, b1, 0) ^ (fp ? ~0ull : 0ull);
-                        // this word's multiplied rows and constants into the list
+                        b1 ^= fp ? ~0ull : 0ull;
                         const u64 Mw = __shfl_sync(kFull, Ml, warp);
                         const int before = __reduce_add_sync(kFull, lane < warp ? __popcll(Ml) : 0);
                         uint16_t *const o = d.mlist + (int64_t)pos * d.list_stride + before;
@@ -371,17 +414,15 @@ __global__ void __launch_bounds__(kWalkThreads, 1) walk_kernel(WalkDev d, int re
                                 o[__popcll(Mw & ((1ull << bit) - 1ull))] =
                                     (uint16_t)((64 * warp + bit) | (((b1 >> bit) & 1ull) ? 0x8000 : 0));
                         }
-                        if (lane == 0 && (mq & kWalkReset))
-                            d.mmask[((int64_t)pos * 2 + 1) * ww + warp] = zc[q * wp + warp];
                         const int rows = __reduce_add_sync(kFull, __popcll(Ml));
                         if (tid == 0)
                             d.minfo[pos] = WalkMeas{1u | (mq & kWalkReset ? 4u : 0u) | (uint32_t)p << 8, rows};
                     }
                     dirty = true;
-                    ci ^= 1;
                     ++pos;
                     continue;
                 }
+                known = false;
                 // deterministic up to e: the next random measurement, or a qubit
                 // that the run has reset
                 {
@@ -416,10 +457,13 @@ __global__ void __launch_bounds__(kWalkThreads, 1) walk_kernel(WalkDev d, int re
                 const int e = min(s_first[fi], c1);
                 fi ^= 1;
                 if (tid == 0) s_first[fi] = 0x7FFFFFFF;  // (every thread is past its last read)
+                const int ts = (2 * n) >> 6;  // the scratch row, which no outcome reads
+                const u64 bs = 1ull << ((2 * n) & 63);
+                if (tid == 0) F[ts] &= ~bs;
                 const int gl = lane & 7;
                 const unsigned gmask = 0xFFu << (lane & 24);
                 const u64 rmd = __shfl_sync(kFull, rm_destab, gl);
-                for (int m = pos + (tid >> 3); m < e; m += kWalkThreads / 8) {
+                for (int m = pos + (tid >> 3) * shares + share; m < e; m += kWalkThreads / 8 * shares) {  // this CTA's share
                     const int32_t v = s_mq[m - c0];
                     const int qm = v & kWalkQubit;
                     const u64 mine = gl < nw ? xc[qm * wp + gl] & rmd : 0ull;  // destabilizer rows, 64 a lane
@@ -452,13 +496,10 @@ __global__ void __launch_bounds__(kWalkThreads, 1) walk_kernel(WalkDev d, int re
                 __syncthreads();
                 // the scratch row is the last one's product, Z on its qubit
                 const int ql = s_mq[e - 1 - c0] & kWalkQubit;
-                const int ts = (2 * n) >> 6;
-                const u64 bs = 1ull << ((2 * n) & 63);
-                if (tid < n) {
-                    xc[tid * wp + ts] &= ~bs;
-                    zc[tid * wp + ts] = (zc[tid * wp + ts] & ~bs) | (tid == ql ? bs : 0ull);
+                for (int j = tid; j < n; j += kWalkThreads) {
+                    xc[j * wp + ts] &= ~bs;
+                    zc[j * wp + ts] = (zc[j * wp + ts] & ~bs) | (j == ql ? bs : 0ull);
                 }
-                if (tid == 0) F[ts] &= ~bs;
                 pos = e;
                 // (the next reads of these words leave the scratch row out, and
                 // a barrier comes before their next write)
@@ -474,8 +515,8 @@ __global__ void __launch_bounds__(kWalkThreads, 1) walk_kernel(WalkDev d, int re
     if (fl) smem_xor64(F + t, fl);
     __syncthreads();
     // pending flips and final bits
-    if (tid < ww) d.fmask[tid] = F[tid];
-    for (int t = warp; t < ww * nw * 2; t += kWalkWarps) {
+    if (share == 0 && tid < ww) d.fmask[tid] = F[tid];
+    for (int t = warp * shares + share; t < ww * nw * 2; t += kWalkWarps * shares) {
         const int pl = t & 1, cb = (t >> 1) % nw, rb = (t >> 1) / nw;
         const u64 *const c = pl ? zc : xc;
         const int q0 = cb * 64 + lane, q1 = q0 + 32;
@@ -717,7 +758,7 @@ int launch_walk_gather(cudaStream_t st, const u64 *X, const u64 *Z, const WalkDe
 int launch_walk(cudaStream_t st, const WalkDev &d, bool reset, cudaGraphConditionalHandle fall) {
     const int rc = allow_max_smem((const void *)walk_kernel);
     if (rc != OK) return rc;
-    walk_kernel<<<1, kWalkThreads, walk_smem_bytes(d.n), st>>>(d, reset ? 1 : 0, fall);
+    walk_kernel<<<kWalkShares, kWalkThreads, walk_smem_bytes(d.n), st>>>(d, reset ? 1 : 0, fall);
     PS_CUDA(cudaGetLastError());
     return OK;
 }

@@ -12,9 +12,9 @@
 //              (row, qubit) is the same in all shots and keeps one bit of
 //              each; if some are not, the rest of the walk does nothing and
 //              the per-shot kernels that follow in the same run do the work;
-//   walk       one CTA takes that one tableau through the whole circuit in
-//              shared memory and writes down what each step means for the
-//              signs, as bit masks over the tableau rows;
+//   walk       a few CTAs take that one tableau through the whole circuit,
+//              each in its shared memory, and write down what each step means
+//              for the signs, as bit masks over the tableau rows;
 //   noise      the sign XORs of the channel outcomes (noise_vec_kernel);
 //   signs      one CTA per shot-word applies the masks to its signs, draws
 //              the random outcomes and writes the records;

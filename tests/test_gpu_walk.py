@@ -128,3 +128,34 @@ def test_tableaux_left_to_the_per_shot_kernels(ps, why, graph):
     (ta, ra), (tb, rb) = out
     assert all(np.array_equal(u, v) for u, v in zip(ta, tb))
     assert all(np.array_equal(u, v) for a, b in zip(ra, rb) for u, v in zip(a, b))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [17, 172, 256, 511])
+def test_long_phases_equal_per_shot_kernels(ps, n):
+    """Phases of more than 512 measurements after deep random layers (pivot
+    rows with Paulis on every column): runs of random ones across the 512 that
+    are held at a time, deterministic ones between them, resets among both."""
+    from plaquette_simulator import circuits as C
+    from plaquette_simulator.circuit import CompiledCircuit
+    rng = np.random.default_rng(n)
+    circ = C.Circuit(n)
+    for _ in range(2):
+        for _ in range(6):
+            for q in range(n):
+                (circ.h, circ.s)[int(rng.integers(2))](q)
+            order = rng.permutation(n)
+            for a, b in zip(order[0::2], order[1::2]):
+                (circ.cx, circ.cz)[int(rng.integers(2))](int(a), int(b))
+        for q in rng.integers(0, n, 2 * n + 600):
+            (circ.r if rng.integers(4) == 0 else circ.m)(int(q))
+    out = []
+    for walk in (True, False):
+        st = ps.CliffordState(n, 70, 5, True)
+        cc = CompiledCircuit(circ, st, shared_xz=walk)
+        cc.run()
+        assert _walked(cc, False) == walk  # (runs it once more)
+        out.append((st.tableau_words(0, st.words()), _records(st, cc, circ.num_measurements())))
+    (ta, ra), (tb, rb) = out
+    assert all(np.array_equal(u, v) for u, v in zip(ta, tb))
+    assert all(np.array_equal(u, v) for a, b in zip(ra, rb) for u, v in zip(a, b))
