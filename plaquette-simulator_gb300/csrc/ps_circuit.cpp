@@ -27,17 +27,47 @@ namespace ps {
 
 namespace {
 
-// Detector d, word k: XOR of the records idx[off[d] .. off[d+1]) (coalesced
-// over words).
-__global__ void detector_kernel(const u64 *__restrict__ res, int64_t w, const uint32_t *__restrict__ idx,
-                                const uint64_t *__restrict__ off, int64_t ndet, u64 *__restrict__ out) {
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < ndet * w;
+// Definitions of detectors as a kernel argument: offsets [ndet + 1], then
+// indices.  Those of the small circuits, whose call is latency, fit (d = 7, 7
+// rounds: 337 + 1,000 or so); an upload in front of the kernel costs 8 us.
+constexpr uint64_t kDetArgs = 1976;
+constexpr size_t kDetKeep = (size_t)64 << 20;
+struct DetArgs {
+    uint16_t v[kDetArgs];
+};
+
+// Detector d, 16 bytes k: XOR of the records idx[off[d] .. off[d+1])
+// (coalesced over words; the reads of one detector do not wait for each
+// other).
+template <class Off, class Idx>
+__device__ __forceinline__ void detector_rows(const u64 *__restrict__ res, int64_t w, const Idx *__restrict__ idx,
+                                              const Off *__restrict__ off, int64_t ndet, u64 *__restrict__ out) {
+    const ulonglong2 *const r2 = reinterpret_cast<const ulonglong2 *>(res);
+    const int64_t half = w >> 1;  // (words are even)
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < ndet * half;
          e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t d = e / w, k = e - d * w;
-        u64 v = 0ull;
-        for (uint64_t j = off[d]; j < off[d + 1]; ++j) v ^= res[(int64_t)idx[j] * w + k];
-        out[e] = v;
+        const int64_t d = e / half, k = e - d * half;
+        ulonglong2 v = make_ulonglong2(0ull, 0ull);
+        const uint64_t j1 = off[d + 1];
+#pragma unroll 4
+        for (uint64_t j = off[d]; j < j1; ++j) {
+            const ulonglong2 r = r2[(int64_t)idx[j] * half + k];
+            v.x ^= r.x;
+            v.y ^= r.y;
+        }
+        reinterpret_cast<ulonglong2 *>(out)[e] = v;
     }
+}
+__global__ void __launch_bounds__(128) detector_kernel(const u64 *__restrict__ res, int64_t w,
+                                                       const uint32_t *__restrict__ idx,
+                                                       const uint64_t *__restrict__ off, int64_t ndet,
+                                                       u64 *__restrict__ out) {
+    detector_rows(res, w, idx, off, ndet, out);
+}
+__global__ void __launch_bounds__(128) detector_args_kernel(const u64 *__restrict__ res, int64_t w,
+                                                            const __grid_constant__ DetArgs a, int64_t ndet,
+                                                            u64 *__restrict__ out) {
+    detector_rows(res, w, a.v + ndet + 1, a.v, ndet, out);
 }
 
 __global__ void set_params_kernel(RunParams *p, uint64_t seed, uint64_t event_base, uint64_t word_base,
@@ -223,6 +253,12 @@ struct ps_circuit {
     cudaEvent_t ev_ran = nullptr, ev_copied = nullptr;
     bool copy_pending = false;
     int32_t *h_err = nullptr;
+    // ps_circuit_detectors: its scratch, kept between calls (up to kDetKeep
+    // bytes; not on a pooled state, whose pool others share).  Its three
+    // allocations and frees were 25 us of a call.
+    std::mutex det_mutex;
+    void *d_det_scratch = nullptr;
+    size_t det_bytes = 0;
     cudaGraph_t graph[2] = {nullptr, nullptr};      // [reset_state]
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
 };
@@ -2540,35 +2576,47 @@ ps_status ps_circuit_detectors(ps_circuit *c, const uint32_t *idx, const uint64_
     for (uint64_t j = 0; j < nidx; ++j)
         if (idx[j] >= nm) return fail(E_RANGE, "detector refers to measurement " + std::to_string(idx[j]) +
                                                    " of a circuit with " + std::to_string(nm));
-    void *d_idx = nullptr, *d_off = nullptr, *d_out = nullptr;
     const size_t out_bytes = (size_t)ndet * (size_t)h->w * sizeof(u64);
-    int rc = dev_alloc(h, &d_idx, std::max<uint64_t>(1, nidx) * sizeof(uint32_t));
-    if (rc == OK) rc = dev_alloc(h, &d_off, (ndet + 1) * sizeof(uint64_t));
-    if (rc == OK) rc = dev_alloc(h, &d_out, out_bytes);
-    auto cleanup = [&] {
-        cudaStreamSynchronize(h->stream);
-        dev_free(h, d_idx);
-        dev_free(h, d_off);
-        dev_free(h, d_out);
-    };
-    if (rc != OK) {
-        cleanup();
-        return rc;
+    const bool args = nm <= 0xFFFFu && ndet < kDetArgs && nidx <= kDetArgs - ndet - 1;
+    const size_t off_bytes = args ? 0 : (ndet + 1) * sizeof(uint64_t), idx_bytes = args ? 0 : nidx * sizeof(uint32_t);
+    const size_t bytes = out_bytes + off_bytes + idx_bytes;
+    std::lock_guard<std::mutex> lock(c->det_mutex);  // (callers on several threads take turns with the scratch)
+    int rc = OK;
+    if (bytes > c->det_bytes) {
+        dev_free(h, c->d_det_scratch);
+        c->d_det_scratch = nullptr;
+        c->det_bytes = 0;
+        rc = dev_alloc(h, &c->d_det_scratch, bytes);
+        if (rc != OK) return rc;
+        c->det_bytes = bytes;
     }
+    char *const b8 = static_cast<char *>(c->d_det_scratch);
+    u64 *const d_out = reinterpret_cast<u64 *>(b8);
+    uint64_t *const d_off = reinterpret_cast<uint64_t *>(b8 + out_bytes);
+    uint32_t *const d_idx = reinterpret_cast<uint32_t *>(b8 + out_bytes + off_bytes);
+    const int64_t work = (int64_t)ndet * (h->w >> 1);
+    const int blocks = (int)std::min<int64_t>((work + 127) / 128, 152 * 16);
     cudaError_t e = cudaSuccess;
-    if (nidx) e = cudaMemcpyAsync(d_idx, idx, nidx * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_off, off, (ndet + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess) {
-        const int64_t work = (int64_t)ndet * h->w;
-        const int blocks = (int)std::min<int64_t>((work + 255) / 256, 152 * 16);
-        detector_kernel<<<blocks, 256, 0, h->stream>>>(c->d_res_block, h->w, (const uint32_t *)d_idx,
-                                                        (const uint64_t *)d_off, (int64_t)ndet, (u64 *)d_out);
-        e = cudaGetLastError();
+    if (args) {
+        DetArgs a;
+        for (uint64_t d = 0; d <= ndet; ++d) a.v[d] = (uint16_t)off[d];
+        for (uint64_t j = 0; j < nidx; ++j) a.v[ndet + 1 + j] = (uint16_t)idx[j];
+        detector_args_kernel<<<blocks, 128, 0, h->stream>>>(c->d_res_block, h->w, a, (int64_t)ndet, d_out);
+    } else {
+        e = cudaMemcpyAsync(d_off, off, off_bytes, cudaMemcpyHostToDevice, h->stream);
+        if (e == cudaSuccess && nidx) e = cudaMemcpyAsync(d_idx, idx, idx_bytes, cudaMemcpyHostToDevice, h->stream);
+        if (e == cudaSuccess)
+            detector_kernel<<<blocks, 128, 0, h->stream>>>(c->d_res_block, h->w, d_idx, d_off, (int64_t)ndet, d_out);
     }
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, d_out, out_bytes, cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cleanup();
+    const cudaError_t es = cudaStreamSynchronize(h->stream);
+    if (e == cudaSuccess) e = es;
+    if (h->pool || c->det_bytes > kDetKeep) {
+        dev_free(h, c->d_det_scratch);
+        c->d_det_scratch = nullptr;
+        c->det_bytes = 0;
+    }
     if (e != cudaSuccess) return cuda_fail(e, "detectors");
     return OK;
 }
@@ -2601,6 +2649,7 @@ ps_status ps_circuit_destroy(ps_circuit *c) {
     if (c->h_err) cudaFreeHost(c->h_err);
     for (void *p : c->owned) dev_free(c->h, p);
     dev_free(c->h, c->d_forced);
+    dev_free(c->h, c->d_det_scratch);
     delete c;
     return OK;
 }

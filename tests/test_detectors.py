@@ -61,3 +61,27 @@ def test_device_detectors_match_records(ps, p):
         assert not _bits(got, shots).any()
     with pytest.raises(Exception):
         cc.detectors([[nm]])  # index past the last measurement
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shots", [1, 130, 1000])
+@pytest.mark.parametrize("ndet,nidx", [(1, 0), (1, 1), (3, 9), (500, 1475), (500, 1476), (1975, 0), (1976, 0), (4000, 9000)])
+def test_detector_definitions_of_any_size(ps, shots, ndet, nidx):
+    """Definitions that travel with the launch (offsets and indices of 1,976
+    words) and those that do not, empty and repeated ones, one circuit's calls
+    growing and shrinking."""
+    from plaquette_simulator import circuits as C
+    from plaquette_simulator.circuit import CompiledCircuit
+    circ = C.surface_code_memory(3, 3, p=1e-2)
+    st = ps.CliffordState(circ.num_qubits, shots, 4, True)
+    cc = CompiledCircuit(circ, st)
+    cc.run(reset=True)
+    nm = circ.num_measurements()
+    res = np.zeros((nm, ((shots + 63) // 64 + 1) & ~1), np.uint64)
+    cc.copy_records_words(res, None)
+    rng = np.random.default_rng(ndet + nidx)
+    cuts = np.sort(rng.integers(0, nidx + 1, ndet - 1))
+    defs = [list(map(int, d)) for d in np.split(rng.integers(0, nm, nidx), cuts)]
+    for some in (defs[:1], defs, defs[-2:]):
+        want = np.stack([np.bitwise_xor.reduce(res[d], axis=0) if d else np.zeros_like(res[0]) for d in some])
+        assert np.array_equal(cc.detectors(some), want)
