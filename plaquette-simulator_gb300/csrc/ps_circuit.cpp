@@ -261,6 +261,7 @@ struct ps_circuit {
     size_t det_bytes = 0;
     cudaGraph_t graph[2] = {nullptr, nullptr};      // [reset_state]
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
+    cudaGraphNode_t pnode[2] = {nullptr, nullptr};  // the run's parameters
 };
 
 namespace ps {
@@ -1677,6 +1678,34 @@ int enqueue_plan(ps_circuit *c, cudaStream_t st, bool reset, Profiler *prof = nu
     return enqueue_steps(c, st, 0, c->steps.size(), prof);
 }
 
+// The run's parameters, as the graph's first node: set in the executable
+// graph before each launch (a launch of its own in front of the graph's cost
+// 3 us more).
+int capture_params(ps_circuit *c, cudaStream_t cs, int reset) {
+    set_params_kernel<<<1, 1, 0, cs>>>(c->d_params, 0, 0, 0, 0);
+    PS_CUDA(cudaGetLastError());
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    const cudaGraphNode_t *deps = nullptr;
+    size_t nd = 0;
+    PS_CUDA(cudaStreamGetCaptureInfo(cs, &status, nullptr, nullptr, &deps, nullptr, &nd));
+    if (nd != 1) return fail(E_CUDA, "capture of the run's parameters");
+    c->pnode[reset] = deps[0];
+    return OK;
+}
+
+int graph_launch(ps_circuit *c, int reset, const RunParams &p) {
+    RunParams *dst = c->d_params;
+    uint64_t seed = p.seed, event_base = p.event_base, word_base = p.word_base, valid = p.valid;
+    void *args[] = {&dst, &seed, &event_base, &word_base, &valid};
+    cudaKernelNodeParams kp = {};
+    kp.func = (void *)set_params_kernel;
+    kp.gridDim = kp.blockDim = dim3(1);
+    kp.kernelParams = args;
+    PS_CUDA(cudaGraphExecKernelNodeSetParams(c->exec[reset], c->pnode[reset], &kp));
+    PS_CUDA(cudaGraphLaunch(c->exec[reset], c->h->stream));
+    return OK;
+}
+
 // Captures the plan of runs without (reset = 0) or with the reset into its
 // CUDA graph, replacing an earlier one.
 int capture_graph(ps_circuit *c, int reset) {
@@ -1687,7 +1716,9 @@ int capture_graph(ps_circuit *c, int reset) {
     cudaStream_t cs;
     PS_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
     cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
-    int rc = e == cudaSuccess ? enqueue_plan(c, cs, reset != 0) : cuda_fail(e, "cudaStreamBeginCapture");
+    int rc = e == cudaSuccess ? OK : cuda_fail(e, "cudaStreamBeginCapture");
+    if (rc == OK) rc = capture_params(c, cs, reset);
+    if (rc == OK) rc = enqueue_plan(c, cs, reset != 0);
     cudaGraph_t g = nullptr;
     cudaError_t e2 = cudaStreamEndCapture(cs, &g);
     cudaStreamDestroy(cs);
@@ -2404,8 +2435,6 @@ ps_status ps_circuit_run(ps_circuit *c, int reset_state) {
     NvtxRange range("ps circuit run");
     if (c->copy_pending) PS_CUDA(cudaStreamWaitEvent(h->stream, c->ev_copied, 0));  // it rewrites those records
     const RunParams p = begin_run(c, reset_state != 0);
-    set_params_kernel<<<1, 1, 0, h->stream>>>(c->d_params, p.seed, p.event_base, p.word_base, p.valid);
-    PS_CUDA(cudaGetLastError());
     if (!reset_state && c->opts.use_graph && !c->exec[0] && c->frame_ok && !h->signs_only &&
         c->seg_dev_status < 0) {
         // the first run without reset of a shared-x/z circuit: build and capture its per-shot plan
@@ -2413,10 +2442,9 @@ ps_status ps_circuit_run(ps_circuit *c, int reset_state) {
         if (rc == OK) rc = capture_graph(c, 0);
         if (rc != OK) return rc;
     }
-    if (c->exec[reset_state ? 1 : 0]) {
-        PS_CUDA(cudaGraphLaunch(c->exec[reset_state ? 1 : 0], h->stream));
-        return OK;
-    }
+    if (c->exec[reset_state ? 1 : 0]) return graph_launch(c, reset_state ? 1 : 0, p);
+    set_params_kernel<<<1, 1, 0, h->stream>>>(c->d_params, p.seed, p.event_base, p.word_base, p.valid);
+    PS_CUDA(cudaGetLastError());
     return enqueue_plan(c, h->stream, reset_state != 0);
 }
 
