@@ -658,6 +658,18 @@ size_t frame_smem_bytes(int64_t n) {  // rows, the zero row, kWinRows sink rows
     return (size_t)(2 * n + 2 + kWinRows) * sizeof(u64);
 }
 
+int beside_broadcast(const void *kernel) { return same_carveout(kernel); }
+
+int broadcast_sms(int *sms) {
+    if (g_frame_sms == 0) {
+        int dev = 0;
+        PS_CUDA(cudaGetDevice(&dev));
+        PS_CUDA(cudaDeviceGetAttribute(&g_frame_sms, cudaDevAttrMultiProcessorCount, dev));
+    }
+    *sms = g_frame_sms;
+    return OK;
+}
+
 int launch_noise_vectors(cudaStream_t st, const FrameTable &t) {
     if (t.njobs <= 0 || t.nctas <= 0) return OK;
     if (t.nsmem > kSegSmemMax) return fail(E_ARG, "channel noise does not fit in shared memory");
@@ -707,10 +719,10 @@ int launch_frame_run(cudaStream_t st, const FrameTable &t, int warps) {
 
 int launch_broadcast_jobs(cudaStream_t st, const FrameTable &t, int ctas_per_sm) {
     if (t.njobs <= 0 || t.chunks <= 0) return OK;
-    if (g_frame_sms == 0) {
-        int dev = 0;
-        PS_CUDA(cudaGetDevice(&dev));
-        PS_CUDA(cudaDeviceGetAttribute(&g_frame_sms, cudaDevAttrMultiProcessorCount, dev));
+    int sms = 0;
+    {
+        int rc = broadcast_sms(&sms);
+        if (rc != OK) return rc;
     }
     {
         int rc = same_carveout((const void *)broadcast_jobs_kernel<true>);
@@ -720,7 +732,7 @@ int launch_broadcast_jobs(cudaStream_t st, const FrameTable &t, int ctas_per_sm)
     int rc = prio_greatest();
     if (rc != OK) return rc;
     const int per = ctas_per_sm > 0 ? ctas_per_sm : 1;
-    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((t.chunks + 7) / 8, (int64_t)g_frame_sms * per));
+    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((t.chunks + 7) / 8, (int64_t)sms * per));
     // The broadcast is the run's longest kernel and its CTAs stay to the
     // end: launched at the highest priority, they reach every SM before the
     // noise and sign CTAs fill them.

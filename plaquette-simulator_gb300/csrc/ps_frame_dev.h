@@ -216,5 +216,9 @@ bool circuit_frame_job(const ps_circuit *c, FrameJobDev *job, BroadcastJobDev *b
 // write at close to the copy rate and leave the noise and sign kernels
 // most of each SM and of the memory system).
 int launch_broadcast_jobs(cudaStream_t st, const FrameTable &t, int ctas_per_sm);
+// Asks for the broadcast's shared-memory carveout, so that a kernel's CTAs
+// can share SMs with it.
+int beside_broadcast(const void *kernel);
+int broadcast_sms(int *sms);  // the device's SMs, one broadcast CTA each
 
 }  // namespace ps

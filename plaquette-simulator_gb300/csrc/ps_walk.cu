@@ -2,6 +2,7 @@
 #include <algorithm>
 
 #include "ps_draw.cuh"
+#include "ps_frame_dev.h"
 #include "ps_walk.h"
 
 namespace ps {
@@ -544,7 +545,13 @@ constexpr int kSignRows = 2;     // tableau rows per thread: 2 * 511 + 1 over 51
 // d = 13, 10,000 shots: 0.12 ms; 90 distillation blocks at 16,384 shots (630
 // random measurements): 0.21 ms, where a barrier and all rows a measurement
 // took 0.41.
-__global__ void __launch_bounds__(kSignThreads, 2) walk_signs_kernel(WalkDev d, int reset) {
+// REGS: two CTAs an SM leave no registers for a broadcast CTA at 64 a thread,
+// and the broadcast, launched first, held the second one off until it was
+// done; at 56 all three fit.  90 blocks, signs and broadcast 422 -> 280 us;
+// where an SM gets one CTA anyway (9 rounds at d = 9, 64 shots) 64 are 2 us
+// better.
+template <int REGS>
+__global__ void __maxnreg__(REGS) walk_signs_kernel(WalkDev d, int reset) {
     extern __shared__ __align__(16) u64 sR[];  // [2n + 1]
     __shared__ u64 sout[kSignChunk];           // drawn outcomes, then outcomes of deterministic measurements
     __shared__ WalkMeas sinfo[kSignChunk];
@@ -764,7 +771,13 @@ int launch_walk(cudaStream_t st, const WalkDev &d, bool reset, cudaGraphConditio
 }
 
 int launch_walk_signs(cudaStream_t st, const WalkDev &d, bool reset) {
-    walk_signs_kernel<<<(unsigned)d.w, kSignThreads, (size_t)(2 * d.n + 1) * sizeof(u64), st>>>(d, reset ? 1 : 0);
+    int sms = 0;
+    int rc = broadcast_sms(&sms);
+    if (rc != OK) return rc;
+    const auto kernel = d.w > sms ? walk_signs_kernel<56> : walk_signs_kernel<64>;
+    rc = beside_broadcast((const void *)kernel);
+    if (rc != OK) return rc;
+    kernel<<<(unsigned)d.w, kSignThreads, (size_t)(2 * d.n + 1) * sizeof(u64), st>>>(d, reset ? 1 : 0);
     PS_CUDA(cudaGetLastError());
     return OK;
 }

@@ -75,7 +75,7 @@ def test_large_registers_equal_per_shot_kernels(ps, n, reset):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("d,rounds,shots", [(3, 4, 200), (5, 3, 4097), (9, 2, 64)])
+@pytest.mark.parametrize("d,rounds,shots", [(3, 4, 200), (5, 3, 4097), (9, 2, 64), (3, 3, 9728), (3, 3, 9729)])
 def test_memory_slices_equal_per_shot_kernels(ps, d, rounds, shots):
     """Noisy rounds run on from a memory's tableau, resets ending the slice
     (applied in their phase) and resets before more gates (deferred)."""
