@@ -1629,18 +1629,30 @@ int enqueue_walk(ps_circuit *c, cudaStream_t st, bool reset, Profiler *prof, cud
     NvtxRange range("ps shared-x/z walk");
     FrameTable t = c->wtable;
     if (reset) t.off = nullptr;
+    const bool beside = !prof && c->fstream, check = !reset && !walk_gathers_all(c->wdev);
     int rc = OK;
     if (!reset) rc = timed(P_INIT, [&] { return launch_walk_gather(st, c->h->X, c->h->Z, c->wdev); });
-    if (rc == OK) rc = timed(P_SEGMENT, [&] { return launch_walk(st, c->wdev, reset, fall); });
     if (rc != OK) return rc;
-    const bool beside = !prof && c->fstream;
+    if (check && beside) {
+        PS_CUDA(cudaEventRecord(c->fev[0], st));
+        PS_CUDA(cudaStreamWaitEvent(c->fstream, c->fev[0], 0));
+        rc = launch_walk_check(c->fstream, c->h->X, c->h->Z, c->wdev);
+        if (rc != OK) return rc;
+        PS_CUDA(cudaEventRecord(c->fev[1], c->fstream));
+    } else if (check) {
+        rc = timed(P_INIT, [&] { return launch_walk_check(st, c->h->X, c->h->Z, c->wdev); });
+        if (rc != OK) return rc;
+    }
+    rc = timed(P_SEGMENT, [&] { return launch_walk(st, c->wdev, reset); });
+    if (rc != OK) return rc;
+    if (check && beside) PS_CUDA(cudaStreamWaitEvent(st, c->fev[1], 0));
     if (beside) {
         PS_CUDA(cudaEventRecord(c->fev[0], st));
         PS_CUDA(cudaStreamWaitEvent(c->fstream, c->fev[0], 0));
         rc = launch_broadcast_jobs(c->fstream, t, c->opts.bcast_ctas);
     }
     if (rc == OK) rc = timed(P_SAMPLE, [&] { return launch_noise_vectors(st, t); });
-    if (rc == OK) rc = timed(P_FRAME, [&] { return launch_walk_signs(st, c->wdev, reset); });
+    if (rc == OK) rc = timed(P_FRAME, [&] { return launch_walk_signs(st, c->wdev, reset, fall); });
     if (rc != OK) return rc;
     if (beside) {
         PS_CUDA(cudaEventRecord(c->fev[1], c->fstream));

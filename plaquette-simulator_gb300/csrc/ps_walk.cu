@@ -49,53 +49,81 @@ __device__ __forceinline__ void transpose64(u64 &a, u64 &b, int lane) {
     }
 }
 
-// ------------------------------------------------------------- gather
-constexpr int kGatherUnroll = 4;  // 16-byte chunks of each plane in flight per thread
-
-// One bit of every (row, qubit), and whether all shots agree on it.  A row
-// of a plane is one stream of 16-byte chunks, `half` of them per qubit; a
-// CTA takes 1,024 consecutive chunks of a row, and a thread compares each
-// with its qubit's first word (in L1: its neighbours read it too), which
-// has to be all zeros or all ones.  The thread of a qubit's first chunk
-// notes the bit (out is zero before).  Bound by the one read of X and Z (d =
-// 15, 16,384 shots: 1.65 GB in 0.27 ms = 6.1 TB/s; a warp per 32 qubits with
-// lanes over each qubit's words: 0.38 ms); a mismatch stops the other CTAs at their next item.
+// ------------------------------------------------------- gather, check
+// The first shot's bit of every (row, qubit): a warp per 32 qubits of a row,
+// which the row's 64-bit words take whole.  The first `words` shot-words have
+// to be all zeros or all ones alike, so shots that differ within them stop
+// the run's walk and check here.  With a small tableau (walk_gathers_all)
+// these are all words, and there is no check: a launch beside the walk costs
+// 4 us (9 rounds at d = 9, 64 shots, 1.7 MB: 176 us instead of 178 a run).
 __global__ void __launch_bounds__(256) walk_gather_kernel(const u64 *__restrict__ X, const u64 *__restrict__ Z, int n,
-                                                         int W, int64_t w, uint32_t *__restrict__ out, int nw,
+                                                         int W, int64_t w, uint32_t *__restrict__ out, int nw, int words,
                                                          int32_t *bad, const RunParams *__restrict__ rp) {
     if (rp->valid == 0) {
         if (blockIdx.x == 0 && threadIdx.x == 0) *bad = 1;
         return;
     }
+    const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // (row, 32 qubits)
+    const int row = (int)(g / (2 * nw)), c = (int)(g - (int64_t)row * 2 * nw), q = 32 * c + (threadIdx.x & 31);
+    if (row >= W) return;
+    u64 x = 0ull, z = 0ull;
+    if (q < n) {
+        x = X[((int64_t)row * n + q) * w];
+        z = Z[((int64_t)row * n + q) * w];
+    }
+    const unsigned bx = __ballot_sync(kFull, x != 0ull), bz = __ballot_sync(kFull, z != 0ull);
+    bool fine = x + 1ull <= 1ull && z + 1ull <= 1ull;
+    if (q < n) {
+        const int64_t at = ((int64_t)row * n + q) * w;
+        for (int k = 1; k < words; ++k) fine &= X[at + k] == x && Z[at + k] == z;
+    }
+    fine = __all_sync(kFull, fine);
+    if ((threadIdx.x & 31) == 0) {
+        out[(int64_t)row * 4 * nw + c] = bx;
+        out[(int64_t)row * 4 * nw + 2 * nw + c] = bz;
+        if (!fine) atomicOr(bad, 1);
+    }
+}
+
+constexpr int kCheckUnroll = 4;  // 16-byte chunks of each plane in flight per thread
+constexpr int kCheckThreads = 1024;
+// One check CTA an SM (more than half of its shared memory): beside the walk,
+// whose CTAs need an SM each, the check takes the other SMs.
+constexpr size_t kCheckSmem = 120 * 1024;
+
+// Whether all shots agree on every (row, qubit).  A row of a plane is one
+// stream of 16-byte chunks, `half` of them per qubit; a CTA takes 4,096
+// consecutive chunks of a row, and a thread compares each with its qubit's
+// first word (in L1: its neighbours read it too), which has to be all zeros
+// or all ones.  Bound by the one read of X and Z (d = 13, 10,000 shots: 0.58 GB
+// in 0.11 ms), which the walk hides where it is the longer one: a run of 13
+// rounds there took 0.53 ms with the check in front of the walk and 0.46
+// beside it.  A mismatch stops the other CTAs at their next item.
+__global__ void __launch_bounds__(kCheckThreads, 1) walk_check_kernel(const u64 *__restrict__ X,
+                                                                      const u64 *__restrict__ Z, int n, int W,
+                                                                      int64_t w, int32_t *bad) {
     const uint32_t half = (uint32_t)(w >> 1), chunks = (uint32_t)n * half;
-    const uint32_t per = 256u * kGatherUnroll, nblk = (chunks + per - 1) / per;
+    const uint32_t per = kCheckThreads * kCheckUnroll, nblk = (chunks + per - 1) / per;
     for (int64_t it = blockIdx.x; it < (int64_t)W * nblk; it += gridDim.x) {
         if (*(volatile int32_t *)bad) return;
         const uint32_t row = (uint32_t)(it / nblk), e0 = ((uint32_t)it - row * nblk) * per + threadIdx.x;
         const u64 *const xr = X + (int64_t)row * n * w, *const zr = Z + (int64_t)row * n * w;
-        ulonglong2 vx[kGatherUnroll], vz[kGatherUnroll];
-        u64 hx[kGatherUnroll], hz[kGatherUnroll];
-        uint32_t q[kGatherUnroll];
+        ulonglong2 vx[kCheckUnroll], vz[kCheckUnroll];
+        u64 hx[kCheckUnroll], hz[kCheckUnroll];
 #pragma unroll
-        for (int u = 0; u < kGatherUnroll; ++u) {
-            const uint32_t e = min(e0 + 256u * u, chunks - 1);  // (past the end: the last chunk again)
-            q[u] = e / half;
+        for (int u = 0; u < kCheckUnroll; ++u) {
+            const uint32_t e = min(e0 + kCheckThreads * u, chunks - 1);  // (past the end: the last chunk again)
+            const uint32_t q = e / half;
             vx[u] = *reinterpret_cast<const ulonglong2 *>(xr + 2ull * e);
             vz[u] = *reinterpret_cast<const ulonglong2 *>(zr + 2ull * e);
-            hx[u] = xr[(int64_t)q[u] * w];
-            hz[u] = zr[(int64_t)q[u] * w];
+            hx[u] = xr[(int64_t)q * w];
+            hz[u] = zr[(int64_t)q * w];
         }
         bool fine = true;
 #pragma unroll
-        for (int u = 0; u < kGatherUnroll; ++u) {
+        for (int u = 0; u < kCheckUnroll; ++u) {
             fine &= vx[u].x == hx[u] && vx[u].y == hx[u] && vz[u].x == hz[u] && vz[u].y == hz[u];
             fine &= hx[u] + 1ull <= 1ull && hz[u] + 1ull <= 1ull;  // all zeros or all ones
-            const uint32_t e = e0 + 256u * u;
-            if (e < chunks && e == q[u] * half) {
-                uint32_t *const o = out + (int64_t)row * 4 * nw + (q[u] >> 5);
-                if (hx[u]) atomicOr(o, 1u << (q[u] & 31u));
-                if (hz[u]) atomicOr(o + 2 * nw, 1u << (q[u] & 31u));
-            }
         }
         if (!fine) atomicOr(bad, 1);
     }
@@ -165,17 +193,15 @@ __host__ __device__ inline WalkSmem walk_layout(int64_t n) {
 // destabilizer rows select, its sign the summed phase of that product;
 // eight lanes take one measurement, a word of the row each, from a
 // row-major copy of the stabilizers that is made again after x / z changed.
-__global__ void __launch_bounds__(kWalkThreads, 1) walk_kernel(WalkDev d, int reset, cudaGraphConditionalHandle fall) {
+__global__ void __launch_bounds__(kWalkThreads, 1) walk_kernel(WalkDev d, int reset) {
     extern __shared__ __align__(16) u64 sm[];
     __shared__ int s_first[2];
     // the next position's pivot (-1: deterministic) and the rows a random one multiplies
     __shared__ int s_pivot[2];
     __shared__ u64 s_rows[2][16];
     __shared__ int32_t s_mq[kWalkThreads];
-    if (!reset && *d.bad) {  // the per-shot kernels' turn (a conditional part of the graph)
-        if (fall && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(fall, 1u);
-        return;
-    }
+    if (!reset && __syncthreads_or(threadIdx.x == 0 && *(volatile int32_t *)d.bad)) return;  // the per-shot kernels' turn
+    const bool poll = !reset && !walk_gathers_all(d);
     const int share = blockIdx.x, shares = gridDim.x;  // which of the outputs this CTA writes
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = d.n, W = 2 * n + 1, ww = d.ww, nw = d.nw, wp = walk_wp(ww), np = walk_np(nw);
@@ -240,6 +266,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) walk_kernel(WalkDev d, int re
     int fi = 0, ci = 0;
     for (int si = 0; si < d.nsteps; ++si) {
         const WalkStep st2 = step(si + 2);
+        const int bad = poll && tid == 0 && st.phase ? *(volatile int32_t *)d.bad : 0;
         const uint32_t hg1 = st1.phase ? 0u : held(d.gates, st1.i0, st1.i1), hs1 = held(d.signs, st1.s0, st1.s1),
                        hn1 = held_slot(st1.n0, st1.n1);
         if (!st.phase) {
@@ -506,7 +533,9 @@ __global__ void __launch_bounds__(kWalkThreads, 1) walk_kernel(WalkDev d, int re
                 // a barrier comes before their next write)
             }
         }
-        if (st.phase) __syncthreads();
+        // (the check beside it may have found shots that differ meanwhile)
+        if (st.phase && poll && __syncthreads_or(bad)) return;
+        if (st.phase && !poll) __syncthreads();
         st = st1;
         st1 = st2;
         hg = hg1;
@@ -551,13 +580,16 @@ constexpr int kSignRows = 2;     // tableau rows per thread: 2 * 511 + 1 over 51
 // where an SM gets one CTA anyway (9 rounds at d = 9, 64 shots) 64 are 2 us
 // better.
 template <int REGS>
-__global__ void __maxnreg__(REGS) walk_signs_kernel(WalkDev d, int reset) {
+__global__ void __maxnreg__(REGS) walk_signs_kernel(WalkDev d, int reset, cudaGraphConditionalHandle fall) {
     extern __shared__ __align__(16) u64 sR[];  // [2n + 1]
     __shared__ u64 sout[kSignChunk];           // drawn outcomes, then outcomes of deterministic measurements
     __shared__ WalkMeas sinfo[kSignChunk];
     __shared__ __align__(4) uint16_t slist[kSignLists * kSignShort];
     __shared__ int snext;
-    if (!reset && *d.bad) return;
+    if (!reset && *d.bad) {  // the per-shot kernels' turn (a conditional part of the graph)
+        if (fall && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(fall, 1u);
+        return;
+    }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = d.n, W = 2 * n + 1, ww = d.ww, nw = d.nw;
     const int64_t w = d.w, k = blockIdx.x;
@@ -739,45 +771,51 @@ __global__ void __maxnreg__(REGS) walk_signs_kernel(WalkDev d, int reset) {
         d.R[(int64_t)i * w + k] = sR[i] ^ (((d.fmask[i >> 6] >> (i & 63)) & 1ull) ? ~0ull : 0ull);
 }
 
-int g_walk_sms = 0;
 
 }  // namespace
 
 size_t walk_smem_bytes(int64_t n) { return walk_layout(n).total; }
 
 int launch_walk_gather(cudaStream_t st, const u64 *X, const u64 *Z, const WalkDev &d) {
-    if (g_walk_sms == 0) {
-        int dev = 0;
-        PS_CUDA(cudaGetDevice(&dev));
-        PS_CUDA(cudaDeviceGetAttribute(&g_walk_sms, cudaDevAttrMultiProcessorCount, dev));
-    }
     const int W = 2 * d.n + 1;
-    // the flag and the bits behind it
-    PS_CUDA(cudaMemsetAsync(d.bad, 0, kWalkCtlBytes + (size_t)W * 2 * (size_t)d.nw * sizeof(uint64_t), st));
-    const int64_t chunks = (int64_t)d.n * (d.w / 2), nblk = (chunks + 256 * kGatherUnroll - 1) / (256 * kGatherUnroll);
-    const int64_t blocks = std::min<int64_t>(W * nblk, (int64_t)g_walk_sms * 4);
-    walk_gather_kernel<<<(unsigned)blocks, 256, 0, st>>>(X, Z, d.n, W, d.w, reinterpret_cast<uint32_t *>(d.gin), d.nw,
-                                                         d.bad, d.rp);
+    PS_CUDA(cudaMemsetAsync(d.bad, 0, kWalkCtlBytes, st));
+    const int64_t warps = (int64_t)W * 2 * d.nw;
+    walk_gather_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(X, Z, d.n, W, d.w,
+                                                                    reinterpret_cast<uint32_t *>(d.gin), d.nw,
+                                                                    walk_gathers_all(d) ? (int)d.w : 1, d.bad, d.rp);
     PS_CUDA(cudaGetLastError());
     return OK;
 }
 
-int launch_walk(cudaStream_t st, const WalkDev &d, bool reset, cudaGraphConditionalHandle fall) {
+int launch_walk_check(cudaStream_t st, const u64 *X, const u64 *Z, const WalkDev &d) {
+    int sms = 0;
+    int rc = broadcast_sms(&sms);
+    if (rc == OK) rc = allow_max_smem((const void *)walk_check_kernel);
+    if (rc != OK) return rc;
+    const int W = 2 * d.n + 1;
+    const int64_t chunks = (int64_t)d.n * (d.w / 2), per = kCheckThreads * kCheckUnroll, nblk = (chunks + per - 1) / per;
+    const int64_t blocks = std::min<int64_t>(W * nblk, std::max(1, sms - kWalkShares));
+    walk_check_kernel<<<(unsigned)blocks, kCheckThreads, kCheckSmem, st>>>(X, Z, d.n, W, d.w, d.bad);
+    PS_CUDA(cudaGetLastError());
+    return OK;
+}
+
+int launch_walk(cudaStream_t st, const WalkDev &d, bool reset) {
     const int rc = allow_max_smem((const void *)walk_kernel);
     if (rc != OK) return rc;
-    walk_kernel<<<kWalkShares, kWalkThreads, walk_smem_bytes(d.n), st>>>(d, reset ? 1 : 0, fall);
+    walk_kernel<<<kWalkShares, kWalkThreads, walk_smem_bytes(d.n), st>>>(d, reset ? 1 : 0);
     PS_CUDA(cudaGetLastError());
     return OK;
 }
 
-int launch_walk_signs(cudaStream_t st, const WalkDev &d, bool reset) {
+int launch_walk_signs(cudaStream_t st, const WalkDev &d, bool reset, cudaGraphConditionalHandle fall) {
     int sms = 0;
     int rc = broadcast_sms(&sms);
     if (rc != OK) return rc;
     const auto kernel = d.w > sms ? walk_signs_kernel<56> : walk_signs_kernel<64>;
     rc = beside_broadcast((const void *)kernel);
     if (rc != OK) return rc;
-    kernel<<<(unsigned)d.w, kSignThreads, (size_t)(2 * d.n + 1) * sizeof(u64), st>>>(d, reset ? 1 : 0);
+    kernel<<<(unsigned)d.w, kSignThreads, (size_t)(2 * d.n + 1) * sizeof(u64), st>>>(d, reset ? 1 : 0, fall);
     PS_CUDA(cudaGetLastError());
     return OK;
 }

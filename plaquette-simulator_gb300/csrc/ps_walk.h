@@ -8,10 +8,12 @@
 // program; the walk covers what it does not: runs without reset, whose
 // starting x / z are on the device only, and circuits with conditional
 // Paulis.  Four launches, whatever the circuit's length:
-//   gather     (runs without reset) reads X and Z once, checks that every
-//              (row, qubit) is the same in all shots and keeps one bit of
-//              each; if some are not, the rest of the walk does nothing and
-//              the per-shot kernels that follow in the same run do the work;
+//   gather     (runs without reset) reads the first shot's bits;
+//   check      (runs without reset, beside the walk; a small tableau's check
+//              is the gather's) reads X and Z once and checks that every (row, qubit) is the same in all shots; if
+//              some are not, the walk ends early, the kernels after it do
+//              nothing and the per-shot kernels that follow in the same run
+//              do the work;
 //   walk       a few CTAs take that one tableau through the whole circuit,
 //              each in its shared memory, and write down what each step means
 //              for the signs, as bit masks over the tableau rows;
@@ -98,11 +100,19 @@ struct WalkDev {
 // The block of `bad`, in front of gin: the flag, the broadcast's counters.
 constexpr size_t kWalkCtlBytes = 256;
 
+// Tableaux that L2 holds easily and of so few shot-words that a thread reads
+// them one after the other are checked whole by the gather.
+constexpr int64_t kWalkGatherBytes = 16 << 20, kWalkGatherWords = 8;
+PS_HD bool walk_gathers_all(const WalkDev &d) {
+    return d.w <= kWalkGatherWords && 16 * (2 * (int64_t)d.n + 1) * d.n * d.w <= kWalkGatherBytes;
+}
+
 size_t walk_smem_bytes(int64_t n);
 int launch_walk_gather(cudaStream_t st, const u64 *X, const u64 *Z, const WalkDev &d);
+int launch_walk_check(cudaStream_t st, const u64 *X, const u64 *Z, const WalkDev &d);
+int launch_walk(cudaStream_t st, const WalkDev &d, bool reset);
 // fall: the condition of the captured graph's per-shot part, set when the
 // walk does not run (0: none).
-int launch_walk(cudaStream_t st, const WalkDev &d, bool reset, cudaGraphConditionalHandle fall);
-int launch_walk_signs(cudaStream_t st, const WalkDev &d, bool reset);
+int launch_walk_signs(cudaStream_t st, const WalkDev &d, bool reset, cudaGraphConditionalHandle fall);
 
 }  // namespace ps

@@ -159,3 +159,31 @@ def test_long_phases_equal_per_shot_kernels(ps, n):
     (ta, ra), (tb, rb) = out
     assert all(np.array_equal(u, v) for u, v in zip(ta, tb))
     assert all(np.array_equal(u, v) for a, b in zip(ra, rb) for u, v in zip(a, b))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("graph", [True, False])
+@pytest.mark.parametrize("n,shots", [(20, 512), (20, 513), (20, 3267), (300, 512)])
+@pytest.mark.parametrize("odd", [0, 70, -1, None])
+def test_check_beside_the_walk(ps, n, shots, odd, graph):
+    """Tableaux of more than eight shot-words or 16 MB (and of eight), whose
+    one odd shot is in the first word, in another or the last: the walk beside
+    the check is dropped for the per-shot kernels, or kept (no odd shot)."""
+    from plaquette_simulator.circuit import CompiledCircuit
+    circ = random_mixed_circuit(n, 300, seed=6, flags=False)
+    out = []
+    for walk in (True, False):
+        st = ps.CliffordState(n, shots, 17, True)
+        forced = np.zeros(shots, np.uint8)
+        if odd is not None:
+            forced[odd] = 1
+        st.apply_hadamard_gate(3)
+        st.measure_qubit(3, forced=forced)
+        st.apply_hadamard_gate_with_apply_flag(7, 0)
+        cc = CompiledCircuit(circ, st, graph=graph, shared_xz=walk)
+        for _ in range(2):
+            cc.run()
+        out.append((st.tableau_words(0, st.words()), _records(st, cc, circ.num_measurements())))
+    (ta, ra), (tb, rb) = out
+    assert all(np.array_equal(u, v) for u, v in zip(ta, tb))
+    assert all(np.array_equal(u, v) for a, b in zip(ra, rb) for u, v in zip(a, b))
