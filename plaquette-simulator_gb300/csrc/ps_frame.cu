@@ -535,11 +535,12 @@ __global__ void __launch_bounds__(256, 8) broadcast_jobs_kernel(const BroadcastJ
     if (off && *off) return;
     const int lane = threadIdx.x & 31;
     if (ctr) {
+        unsigned long long b = 0;
+        if (lane == 0) b = atomicAdd(ctr, 1ull);
         for (;;) {
-            unsigned long long b = 0;
-            if (lane == 0) b = atomicAdd(ctr, 1ull);
             const int64_t base = (int64_t)__shfl_sync(0xFFFFFFFFu, b, 0) * kBcastBatch;
             if (base >= chunks) break;
+            if (lane == 0) b = atomicAdd(ctr, 1ull);
             const int64_t end = base + kBcastBatch < chunks ? base + kBcastBatch : chunks;
             int64_t c = base;
             while (c < end) {  // the batch's chunks, job by job
