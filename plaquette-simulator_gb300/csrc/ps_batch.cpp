@@ -306,6 +306,7 @@ ps_status ps_batch_create(const ps_job_desc *jobs, uint64_t njobs, const ps_batc
         std::vector<FrameJobDev> fj;
         std::vector<BroadcastJobDev> bj;
         std::vector<int64_t> cta0{0}, ncta0{0}, chunk0{0};
+        int64_t pairs = 0;
         for (size_t j : b->order) {
             FrameJobDev job{};
             BroadcastJobDev bjob{};
@@ -315,9 +316,16 @@ ps_status ps_batch_create(const ps_job_desc *jobs, uint64_t njobs, const ps_batc
             fj.push_back(job);
             bj.push_back(bjob);
             cta0.push_back(cta0.back() + job.w);
-            ncta0.push_back(ncta0.back() + (int64_t)job.nnv * job.w);
             chunk0.push_back(chunk0.back() + broadcast_chunks(job.n, job.w));
             b->table.smem = std::max(b->table.smem, frame_job_smem(job));
+            pairs += (int64_t)job.nnv * job.w;
+        }
+        b->table.noise_own = pairs > 0;
+        for (const FrameJobDev &job : fj)
+            if (job.nnv > 0 && noise_units(job, pairs) == 1) b->table.noise_own = false;
+        for (FrameJobDev &job : fj) {
+            job.noise_units = b->table.noise_own ? kNoiseWarps : 1;
+            ncta0.push_back(ncta0.back() + noise_ctas(job));
             if (job.nnv > 0) b->table.nsmem = std::max(b->table.nsmem, noise_job_smem(job));
         }
         if (!fj.empty()) {

@@ -1179,6 +1179,7 @@ int frame_job_ranges(ps_circuit *c, const FrameProgram &P, FrameJobDev &job, std
     job.n_surv = (uint32_t)surv.size();
     job.nnv = (int32_t)nv_range.size();
     job.stage_tabs = (size_t)job.n_ctab * sizeof(FrameChanTab) + (size_t)job.n_thr * 8 + (size_t)job.n_surv * 4 <= kFrameTabStage ? 1u : 0u;
+    job.noise_units = noise_units(job, (int64_t)job.nnv * job.w);
     // staging: drop the largest staged range until the buffers fit, each
     // within kFrameStageMax and both within what the rest of the sign
     // kernel's shared memory leaves
@@ -1435,7 +1436,7 @@ int build_walk(ps_circuit *c) {
         d.nvec = job.nvec;
         d.nvec_rows = frame_wp(h->n);
         const std::vector<FrameJobDev> jobs{job};
-        const std::vector<int64_t> ncta0{0, (int64_t)nv * h->w};
+        const std::vector<int64_t> ncta0{0, noise_ctas(job)};
         FrameJobDev *dj;
         int64_t *dn;
         if (upload(h, c->owned, jobs, &dj) || upload(h, c->owned, ncta0, &dn)) return E_NOMEM;
@@ -1443,6 +1444,7 @@ int build_walk(ps_circuit *c) {
         t.ncta0 = dn;
         t.nctas = ncta0[1];
         t.nsmem = noise_job_smem(job);
+        t.noise_own = job.noise_units > 1;
     }
     const std::vector<BroadcastJobDev> bjobs{{h->X, h->Z, d.xz, h->n, h->w, (int64_t)d.nw}};
     const std::vector<int64_t> chunk0{0, broadcast_chunks(h->n, h->w)};
@@ -2304,7 +2306,7 @@ ps_status ps_circuit_compile(ps_state *h, const ps_op *ops_in, uint64_t nops, co
                 const std::vector<FrameJobDev> jobs{job};
                 const std::vector<BroadcastJobDev> bjobs{bj};
                 const std::vector<int64_t> cta0{0, h->w}, chunk0{0, broadcast_chunks(h->n, h->w)},
-                    ncta0{0, (int64_t)job.nnv * h->w};
+                    ncta0{0, noise_ctas(job)};
                 FrameJobDev *dj = nullptr;
                 BroadcastJobDev *db = nullptr;
                 int64_t *dc = nullptr, *dk = nullptr, *dn = nullptr;
@@ -2322,6 +2324,7 @@ ps_status ps_circuit_compile(ps_state *h, const ps_op *ops_in, uint64_t nops, co
                 c->ftable.chunks = h->signs_only ? 0 : chunk0[1];  // signs only: no x / z to write
                 c->ftable.smem = frame_job_smem(job);
                 c->ftable.nsmem = job.nnv > 0 ? noise_job_smem(job) : 0;
+                c->ftable.noise_own = job.noise_units > 1;
                 c->fjob = job;
                 c->fbjob = bj;
                 if (!h->signs_only && cudaStreamCreateWithFlags(&c->fstream, cudaStreamNonBlocking) != cudaSuccess)

@@ -76,39 +76,47 @@ __device__ __forceinline__ int job_of(const int64_t *__restrict__ first, int njo
 // found by binary search, tables behind generic pointers and S_64 words and
 // records loaded where they are needed it took 1.79 and 3.2.  At d = 15, p =
 // 1e-3, 16,384 shots: 0.065 and 0.085, before 0.090 and 0.176.
-template <int NW, bool MASKS>
+// OWN: a warp per (range, shot-word) instead of a CTA (noise_units).
+template <int NW, bool MASKS, bool OWN>
 __global__ void __launch_bounds__(32 * NW, 32 / NW) noise_vec_kernel(const FrameJobDev *__restrict__ jobs, int njobs,
                                                             const int64_t *__restrict__ ncta0,
                                                             const int32_t *__restrict__ off) {
     extern __shared__ __align__(16) u64 sm[];
     if (MASKS && off && *off) return;
-    constexpr int NT = 32 * NW;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int nw = OWN ? 1 : NW, NT = 32 * nw;  // the pair's warps
+    const int wid = OWN ? 0 : warp, tid = 32 * wid + lane;
     const int j = njobs > 1 ? job_of(ncta0, njobs, (int64_t)blockIdx.x) : 0;
     const FrameJobDev &J = jobs[j];
     const int64_t w = J.w, Wp = frame_wp(J.n);
-    const int64_t local = (int64_t)blockIdx.x - ncta0[j];
-    const int64_t v = local / w, k = local - v * w;
+    const int64_t local = OWN ? ((int64_t)blockIdx.x - ncta0[j]) * NW + warp : (int64_t)blockIdx.x - ncta0[j];
+    const int64_t v = OWN ? min(local / w, (int64_t)J.nnv - 1) : local / w, k = local - v * w;  // (k >= w: past the last pair)
+    auto sync = [&] {
+        if (OWN) __syncwarp();
+        else __syncthreads();
+    };
     const FrameRangeDev L = J.ranges[J.nv_range[v]];
     const NoiseSmem SL = noise_smem_layout(J);
     char *const sb8 = reinterpret_cast<char *>(sm);
-    u64 *const acc = sm;
-    uint32_t *const shit = reinterpret_cast<uint32_t *>(sb8 + SL.hit);  // hit channels: count, then (channel, first draw)
+    u64 *const acc = sm + (OWN ? warp * Wp : 0);
+    uint32_t *const shit =  // hit channels: count, then (channel, first draw)
+        reinterpret_cast<uint32_t *>(sb8 + SL.hit) + (OWN ? (size_t)warp * (2 * J.max_slots + 2) : 0);
     uint32_t *const shitl = shit + 2;
-    u64 *const qf = reinterpret_cast<u64 *>(sb8 + SL.qf) + 128 * wid;        // this warp's queue: shots ...
-    uint2 *const qd = reinterpret_cast<uint2 *>(sb8 + SL.qd) + 128 * wid;    // ... first row entry and count
+    u64 *const qf = reinterpret_cast<u64 *>(sb8 + SL.qf) + 128 * warp;        // this warp's queue: shots ...
+    uint2 *const qd = reinterpret_cast<uint2 *>(sb8 + SL.qd) + 128 * warp;    // ... first row entry and count
     const RunParams rp = *J.rp;
     FrameChanTab *const sctab = reinterpret_cast<FrameChanTab *>(sb8 + SL.tabs);
     uint64_t *const sthr = reinterpret_cast<uint64_t *>(sctab + J.n_ctab);
     uint32_t *const ssurv = reinterpret_cast<uint32_t *>(sthr + J.n_thr);
     if (J.stage_tabs) {
-        for (uint32_t i = tid; i < J.n_ctab; i += NT) sctab[i] = J.ctab[i];
-        for (uint32_t i = tid; i < J.n_thr; i += NT) sthr[i] = J.thr[i];
-        for (uint32_t i = tid; i < J.n_surv; i += NT) ssurv[i] = J.surv[i];
+        for (uint32_t i = threadIdx.x; i < J.n_ctab; i += 32 * NW) sctab[i] = J.ctab[i];
+        for (uint32_t i = threadIdx.x; i < J.n_thr; i += 32 * NW) sthr[i] = J.thr[i];
+        for (uint32_t i = threadIdx.x; i < J.n_surv; i += 32 * NW) ssurv[i] = J.surv[i];
     }
     for (int64_t i = tid; i < Wp; i += NT) acc[i] = 0ull;
     if (tid == 0) *shit = 0u;
-    __syncthreads();
+    __syncthreads();  // (the tables are the CTA's)
+    if (OWN && k >= w) return;
     const uint32_t *const s64 = J.slot_s64 + L.s64_base;
     const FrameSlotDev *const rec = J.slot + L.rec_base;
     auto append = [&](bool hit, uint32_t slot, uint32_t u) {  // warp-aggregated; every lane calls it
@@ -146,14 +154,38 @@ __global__ void __launch_bounds__(32 * NW, 32 / NW) noise_vec_kernel(const Frame
             fetch(g + NT);
             const u32x4 blk =
                 draw_block(rp.seed, g0 + (uint64_t)g, rp.word_base + (uint64_t)k, 0u, TAG_NOISE_FIRST);
+            if (!OWN) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int32_t sl = 4 * g + c + off0;
+                    append(sl >= 0 && sl < L.nslots && blk.v[c] >= now[c], (uint32_t)sl, blk.v[c]);
+                }
+                continue;
+            }
+            // one atomic for the four: here the chain of them is what counts
+            uint32_t hit = 0u, all[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int32_t sl = 4 * g + c + off0;
-                append(sl >= 0 && sl < L.nslots && blk.v[c] >= now[c], (uint32_t)sl, blk.v[c]);
+                const bool on = sl >= 0 && sl < L.nslots && blk.v[c] >= now[c];
+                all[c] = __ballot_sync(0xffffffffu, on);
+                hit |= on ? 1u << c : 0u;
+            }
+            uint32_t at = 0u;
+            if (lane == 0) at = atomicAdd(shit, (uint32_t)(__popc(all[0]) + __popc(all[1]) + __popc(all[2]) + __popc(all[3])));
+            at = __shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                if ((hit >> c) & 1u) {
+                    const uint32_t to = at + __popc(all[c] & ((1u << lane) - 1u));
+                    shitl[2 * to] = (uint32_t)(4 * g + c + off0);
+                    shitl[2 * to + 1] = blk.v[c];
+                }
+                at += __popc(all[c]);
             }
         }
     }
-    __syncthreads();
+    sync();
     // The hits, 32 at a time per warp: a lane per hit samples its word and
     // flips the rows of each component it found (X or Z on a or b, one or two
     // for most hits) that are in the channel's record.  Components with more
@@ -171,7 +203,7 @@ __global__ void __launch_bounds__(32 * NW, 32 / NW) noise_vec_kernel(const Frame
     auto fetch_rec = [&](uint32_t h) {
         if (h < nhit) dn = rec[shitl[2 * h]];
     };
-    const uint32_t h0 = (uint32_t)lane * NW + (uint32_t)wid;  // spread over the warps
+    const uint32_t h0 = (uint32_t)(lane * nw + wid);  // spread over the warps
     fetch_rec(h0);
     for (uint32_t c0 = 0; c0 + (uint32_t)wid < nhit; c0 += NT) {
         const uint32_t h = c0 + h0;
@@ -257,7 +289,7 @@ __global__ void __launch_bounds__(32 * NW, 32 / NW) noise_vec_kernel(const Frame
         }
         __syncwarp();  // the queue applied before it is filled again
     }
-    __syncthreads();
+    sync();
     u64 *const out = J.nvec + ((int64_t)v * w + k) * Wp;
     for (int64_t i = tid; i < Wp; i += NT) out[i] = acc[i];
 }
@@ -678,14 +710,14 @@ int launch_noise_vectors(cudaStream_t st, const FrameTable &t) {
     // CTAs (16K registers) find room beside them.
     const size_t smem = std::max<size_t>(t.nsmem, kNoiseSmemFloor);
     if (t.nctas > 0x7FFFFFFFll) return fail(E_ARG, "channel noise: too many (range, shot-word) pairs in one launch");
-    const void *kern = t.masks ? (const void *)noise_vec_kernel<kNoiseWarps, true>
-                               : (const void *)noise_vec_kernel<kNoiseWarps, false>;
+    const auto kern = t.masks ? (t.noise_own ? noise_vec_kernel<kNoiseWarps, true, true> : noise_vec_kernel<kNoiseWarps, true, false>)
+                              : (t.noise_own ? noise_vec_kernel<kNoiseWarps, false, true> : noise_vec_kernel<kNoiseWarps, false, false>);
     cudaLaunchConfig_t cfg;
     if (smem > 48 * 1024) {
-        const int rc = allow_max_smem(kern);
+        const int rc = allow_max_smem((const void *)kern);
         if (rc != OK) return rc;
     }
-    int rc = same_carveout(kern);
+    int rc = same_carveout((const void *)kern);
     if (rc == OK) rc = prio_greatest();
     if (rc != OK) return rc;
     cfg = {};
@@ -698,10 +730,7 @@ int launch_noise_vectors(cudaStream_t st, const FrameTable &t) {
     attr[0].val.priority = g_prio_least;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (t.masks)
-        PS_CUDA(cudaLaunchKernelEx(&cfg, noise_vec_kernel<kNoiseWarps, true>, t.jobs, (int)t.njobs, t.ncta0, t.off));
-    else
-        PS_CUDA(cudaLaunchKernelEx(&cfg, noise_vec_kernel<kNoiseWarps, false>, t.jobs, (int)t.njobs, t.ncta0, t.off));
+    PS_CUDA(cudaLaunchKernelEx(&cfg, kern, t.jobs, (int)t.njobs, t.ncta0, t.off));
     PS_CUDA(cudaGetLastError());
     return OK;
 }

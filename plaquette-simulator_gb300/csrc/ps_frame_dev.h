@@ -79,7 +79,8 @@ struct FrameJobDev {
     // channels of the largest segment, channel tables (ctab entries, thr
     // words, surv words; staged when stage_tabs = 1)
     uint32_t max_rand, stage_u32, max_ops, max_scratch, max_slots;
-    uint32_t n_ctab, n_thr, n_surv, stage_tabs, pad2;
+    uint32_t n_ctab, n_thr, n_surv, stage_tabs;
+    uint32_t noise_units;  // (range, shot-word) pairs a noise CTA takes: 1, or one a warp
     int32_t *err;  // set to kFrameErrWait when a bounded wait gave up (the run's results are void)
     // Noise vectors: for the nnv ranges with channels (range index
     // nv_range[v]), the XOR that the range's channel outcomes make on the
@@ -133,25 +134,43 @@ constexpr int kNoiseWarps = 4;
 // keeps it to six CTAs an SM.
 constexpr size_t kNoiseSmemFloor = 36 * 1024;
 
-// Shared-memory layout of the noise kernel for one job: the noise vector
-// being summed (Wp words), each warp's queue of hit components (their shots
-// [128], then rows and counts [128]), the channel tables when staged, the hit
-// list (count, then channel and first draw of each hit).
+// Shared-memory layout of the noise kernel for one job: the noise vectors
+// being summed (Wp words each), each warp's queue of hit components (their
+// shots [128], then rows and counts [128]), the channel tables when staged,
+// the hit lists (count, then channel and first draw of each hit).
 struct NoiseSmem {
     size_t qf, qd, tabs, hit, total;
 };
 __host__ __device__ inline NoiseSmem noise_smem_layout(const FrameJobDev &j) {
     NoiseSmem L;
-    L.qf = (size_t)frame_wp(j.n) * 8;
+    L.qf = (size_t)frame_wp(j.n) * 8 * j.noise_units;
     L.qd = L.qf + (size_t)kNoiseWarps * 128 * 8;
     L.tabs = L.qd + (size_t)kNoiseWarps * 128 * 8;
     L.hit = frame_align16(L.tabs + (j.stage_tabs ? (size_t)j.n_ctab * sizeof(FrameChanTab) + (size_t)j.n_thr * 8 +
                                                        (size_t)j.n_surv * 4
                                                  : 0));
-    L.total = L.hit + (size_t)(2 * j.max_slots + 2) * 4;
+    L.total = L.hit + (size_t)(2 * j.max_slots + 2) * 4 * j.noise_units;
     return L;
 }
 inline size_t noise_job_smem(const FrameJobDev &j) { return noise_smem_layout(j).total; }
+inline int64_t noise_ctas(const FrameJobDev &j) {
+    return ((int64_t)j.nnv * j.w + j.noise_units - 1) / j.noise_units;
+}
+// How many (range, shot-word) pairs a noise CTA takes, in a launch of `pairs`
+// of them.  The channels of a short range keep one warp busy, not four, and
+// its CTA is a chain of loads: where there are pairs enough to fill the chip
+// with six CTAs an SM, a warp each hides four times as much of it.  One kernel
+// per launch: a table whose jobs are not all short keeps a CTA a pair (a
+// kernel of both forms was 1 to 2 % slower at d = 15 and d = 21).  Measured, a
+// run with a CTA and with a warp a pair: d = 3, 60,000 shots, p = 5e-3 56 and
+// 47 us; d = 7, 30,000 shots, p = 1e-3 82 and 67; eight jobs up to d = 9 (430
+// channels a range) 170 and 133.
+constexpr uint32_t kNoiseWarpSlots = 512;
+constexpr int64_t kNoiseWarpPairs = 6 * 152;
+inline uint32_t noise_units(FrameJobDev j, int64_t pairs) {
+    j.noise_units = kNoiseWarps;
+    return j.max_slots <= kNoiseWarpSlots && pairs > kNoiseWarpPairs && noise_job_smem(j) <= kNoiseSmemFloor ? kNoiseWarps : 1;
+}
 
 // One job of the x / z broadcast: X and Z of every (row, qubit) pair and
 // shot-word := the shared bits xz ([W][2][nw64]).
@@ -188,6 +207,7 @@ struct FrameTable {
     // count; zero again after every launch); null: a static chunk split
     unsigned long long *bctr = nullptr;
     bool masks = false;            // the channels' rows are masks (FrameJobDev::smask)
+    bool noise_own = false;  // the noise kernel's pairs are a warp's (noise_units)
     const int32_t *off = nullptr;  // not 0 on the device: noise and broadcast launches do nothing
 };
 // Broadcast chunks a warp takes from the counter at a time.

@@ -1,0 +1,71 @@
+"""Noise CTAs that take a (range, shot-word) pair a warp: launches with more
+than 912 pairs of at most 512 channels, against the per-shot kernels (which
+draw every channel by itself), alone and in a table of jobs; a last CTA with
+idle warps, and the sizes next to both limits."""
+import numpy as np
+import pytest
+
+
+def _outputs(cc, st, circ):
+    st.synchronize()
+    w = ((st.get_batch_size() + 63) // 64 + 1) & ~1
+    res = np.zeros((circ.num_measurements(), w), np.uint64)
+    det = np.zeros_like(res)
+    cc.copy_records_words(res, det)
+    return res, det, st.tableau_words(0, st.words())
+
+
+# 912 pairs and more, of 50 channels each; ragged words (a last CTA with idle
+# warps); ranges of 500, 512 and 513 channels
+@pytest.mark.gpu
+@pytest.mark.parametrize("ranges,channels,shots", [(3, 50, 64 * 304), (3, 50, 64 * 306), (5, 7, 20001),
+                                                   (4, 500, 20000), (1, 512, 64 * 914), (1, 513, 64 * 914)])
+def test_pairs_of_a_warp_equal_per_shot_kernels(ps, ranges, channels, shots):
+    from plaquette_simulator import circuits as C
+    from plaquette_simulator.circuit import CompiledCircuit
+    n = 9
+    rng = np.random.default_rng(channels)
+    circ = C.Circuit(n)
+    for r in range(ranges):
+        for q in range(n):
+            (circ.h, circ.s)[int(rng.integers(2))](q)
+        for a, b in zip(range(0, n - 1, 2), range(1, n, 2)):
+            circ.cx(a, b)
+        for k in range(channels):
+            if k % 3 == 0:
+                a, b = (int(x) for x in rng.choice(n, 2, replace=False))
+                circ.pauli2(a, b, [0.002] * 15)
+            else:
+                circ.pauli1(int(rng.integers(n)), 0.01, 0.02, 0.0)
+        for q in rng.choice(n, 3, replace=False):
+            circ.m(int(q))
+    out = []
+    for shared in (True, False):
+        st = ps.CliffordState(n, shots, 29, True)
+        cc = CompiledCircuit(circ, st, shared_xz=shared)
+        assert bool(cc.stats["shared_xz"]) == shared
+        cc.run(reset=True)
+        cc.run(reset=True)
+        out.append(_outputs(cc, st, circ))
+    (ra, da, ta), (rb, db, tb) = out
+    assert np.array_equal(ra, rb) and np.array_equal(da, db)
+    assert all(np.array_equal(u, v) for u, v in zip(ta, tb))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [[(3, 20000), (5, 7001), (3, 64), (7, 130)], [(3, 20000), (11, 200)]])
+def test_tables_of_jobs_equal_jobs_alone(ps, sizes):
+    """Tables whose ranges are all short, and one that holds a long one."""
+    from plaquette_simulator import circuits as C
+    from plaquette_simulator.batch import Batch, Job
+    from plaquette_simulator.circuit import CompiledCircuit
+    jobs = [Job(C.surface_code_memory(d, 3, p=5e-3), shots, 100 + i) for i, (d, shots) in enumerate(sizes)]
+    batch = Batch(jobs)
+    batch.run()
+    for i, job in enumerate(jobs):
+        res, det = batch.records(i)
+        st = ps.CliffordState(job.circuit.num_qubits, job.shots, job.seed, True)
+        cc = CompiledCircuit(job.circuit, st, shared_xz=False)
+        cc.run(reset=True)
+        want, wdet, _ = _outputs(cc, st, job.circuit)
+        assert np.array_equal(res, want) and np.array_equal(det, wdet)
