@@ -317,6 +317,7 @@ ps_status ps_batch_create(const ps_job_desc *jobs, uint64_t njobs, const ps_batc
             bj.push_back(bjob);
             cta0.push_back(cta0.back() + job.w);
             chunk0.push_back(chunk0.back() + broadcast_chunks(job.n, job.w));
+            b->table.cells += broadcast_cells(job.n, job.w);
             b->table.smem = std::max(b->table.smem, frame_job_smem(job));
             pairs += (int64_t)job.nnv * job.w;
         }

@@ -1454,6 +1454,7 @@ int build_walk(ps_circuit *c) {
     t.bjobs = db;
     t.chunk0 = dk;
     t.chunks = chunk0[1];
+    t.cells = broadcast_cells(h->n, h->w);
     if (!c->fstream && cudaStreamCreateWithFlags(&c->fstream, cudaStreamNonBlocking) != cudaSuccess)
         return cuda_fail(cudaGetLastError(), "cudaStreamCreate");
     for (cudaEvent_t &e : c->fev)
@@ -2321,6 +2322,7 @@ ps_status ps_circuit_compile(ps_state *h, const ps_op *ops_in, uint64_t nops, co
                 c->ftable.njobs = 1;
                 c->ftable.ctas = h->w;
                 c->ftable.nctas = ncta0[1];
+                c->ftable.cells = broadcast_cells(h->n, h->w);
                 c->ftable.chunks = h->signs_only ? 0 : chunk0[1];  // signs only: no x / z to write
                 c->ftable.smem = frame_job_smem(job);
                 c->ftable.nsmem = job.nnv > 0 ? noise_job_smem(job) : 0;

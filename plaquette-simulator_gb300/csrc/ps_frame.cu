@@ -554,15 +554,16 @@ __device__ __forceinline__ void broadcast_chunk(const BroadcastJobDev &B, int64_
 // thread: two broadcast CTAs (16K registers) fit on an SM beside six noise
 // CTAs (48K) or two sign CTAs (40K).
 //
-// With a counter (ctr), warps take kBcastBatch chunks at a time from it, so
-// CTAs that reach their SMs late (beside the other kernels of the run) take
+// With a counter (ctr), warps take `batch` chunks at a time from it, the next
+// ones while they store (the atomic's answer was an eighth of the time of
+// narrow jobs: eight jobs up to d = 15 417 us, asked ahead 364), so CTAs that reach their SMs late (beside the other kernels of the run) take
 // less of the work; the last CTA to finish puts the counter back to zero
 // for the next launch.  Without one, warp i takes chunks i, i + warps, ...
 // ONE: a table of one job (no job lookup).
 template <bool ONE>
 __global__ void __launch_bounds__(256, 8) broadcast_jobs_kernel(const BroadcastJobDev *__restrict__ jobs, int njobs,
                                                              const int64_t *__restrict__ chunk0, int64_t chunks,
-                                                             unsigned long long *ctr,
+                                                             int batch, unsigned long long *ctr,
                                                              const int32_t *__restrict__ off) {
     if (off && *off) return;
     const int lane = threadIdx.x & 31;
@@ -570,10 +571,10 @@ __global__ void __launch_bounds__(256, 8) broadcast_jobs_kernel(const BroadcastJ
         unsigned long long b = 0;
         if (lane == 0) b = atomicAdd(ctr, 1ull);
         for (;;) {
-            const int64_t base = (int64_t)__shfl_sync(0xFFFFFFFFu, b, 0) * kBcastBatch;
+            const int64_t base = (int64_t)__shfl_sync(0xFFFFFFFFu, b, 0) * batch;
             if (base >= chunks) break;
             if (lane == 0) b = atomicAdd(ctr, 1ull);
-            const int64_t end = base + kBcastBatch < chunks ? base + kBcastBatch : chunks;
+            const int64_t end = base + batch < chunks ? base + batch : chunks;
             int64_t c = base;
             while (c < end) {  // the batch's chunks, job by job
                 const int j = ONE ? 0 : job_of(chunk0, njobs, c);
@@ -776,10 +777,11 @@ int launch_broadcast_jobs(cudaStream_t st, const FrameTable &t, int ctas_per_sm)
     attr[0].val.priority = g_prio_greatest;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    const int batch = broadcast_batch(t.cells, t.chunks);
     if (t.njobs == 1)
-        PS_CUDA(cudaLaunchKernelEx(&cfg, broadcast_jobs_kernel<true>, t.bjobs, (int)t.njobs, t.chunk0, t.chunks, t.bctr, t.off));
+        PS_CUDA(cudaLaunchKernelEx(&cfg, broadcast_jobs_kernel<true>, t.bjobs, (int)t.njobs, t.chunk0, t.chunks, batch, t.bctr, t.off));
     else
-        PS_CUDA(cudaLaunchKernelEx(&cfg, broadcast_jobs_kernel<false>, t.bjobs, (int)t.njobs, t.chunk0, t.chunks, t.bctr, t.off));
+        PS_CUDA(cudaLaunchKernelEx(&cfg, broadcast_jobs_kernel<false>, t.bjobs, (int)t.njobs, t.chunk0, t.chunks, batch, t.bctr, t.off));
     PS_CUDA(cudaGetLastError());
     return OK;
 }

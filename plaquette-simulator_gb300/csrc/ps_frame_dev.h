@@ -188,6 +188,7 @@ inline int64_t broadcast_chunks(int64_t n, int64_t w) {
     const int64_t per = 32 / (hw > 0 ? hw : 1);
     return (pairs + per - 1) / per;
 }
+inline int64_t broadcast_cells(int64_t n, int64_t w) { return (2 * n + 1) * n * (w / 2); }
 
 // A table of jobs on the device: jobs[njobs], cta0[njobs + 1] (first CTA of
 // each job in the sign kernel, prefix sums of w), ncta0[njobs + 1] (first CTA
@@ -201,6 +202,7 @@ struct FrameTable {
     const int64_t *chunk0 = nullptr;
     int32_t njobs = 0;
     int64_t ctas = 0, nctas = 0, chunks = 0;  // totals
+    int64_t cells = 0;                        // 16-byte cells of a plane, all jobs
     size_t smem = 0;                          // largest frame_job_smem of the table
     size_t nsmem = 0;                         // largest noise_job_smem of the table
     // two zeroed words (the broadcast's chunk counter and finished-CTA
@@ -210,8 +212,16 @@ struct FrameTable {
     bool noise_own = false;  // the noise kernel's pairs are a warp's (noise_units)
     const int32_t *off = nullptr;  // not 0 on the device: noise and broadcast launches do nothing
 };
-// Broadcast chunks a warp takes from the counter at a time.
-constexpr int64_t kBcastBatch = 8;
+// Broadcast chunks a warp takes from the counter at a time.  What a warp
+// writes as one stream is best near 16 KB of a plane: with 128 cells a chunk
+// eight chunks (d = 15, 16,384 shots: 255 us a run, sixteen 274), with fewer
+// sixteen (d = 23, 13 rounds, 13,000 shots, 102 cells: 1,195 and 1,080 us; d =
+// 21, 10 rounds, 9,000 shots 596 and 529; d = 17, 3 rounds, 5,000 shots 215 and
+// 185; beside more noise, d = 19, 19 rounds, 12,000 shots, 484 and 497).  Tables
+// that would leave a warp of the 152 SMs less than four turns keep eight.
+inline int broadcast_batch(int64_t cells, int64_t chunks) {
+    return cells >= 128 * chunks || chunks < 64 * 8 * 152 ? 8 : 16;
+}
 
 // The noise vectors of every job (nothing when no job has channels).
 int launch_noise_vectors(cudaStream_t st, const FrameTable &t);
