@@ -1179,7 +1179,7 @@ int frame_job_ranges(ps_circuit *c, const FrameProgram &P, FrameJobDev &job, std
     job.n_surv = (uint32_t)surv.size();
     job.nnv = (int32_t)nv_range.size();
     job.stage_tabs = (size_t)job.n_ctab * sizeof(FrameChanTab) + (size_t)job.n_thr * 8 + (size_t)job.n_surv * 4 <= kFrameTabStage ? 1u : 0u;
-    job.noise_units = noise_units(job, (int64_t)job.nnv * job.w);
+    job.noise_units = noise_units(job, (int64_t)job.nnv * job.w, max_slots);
     // staging: drop the largest staged range until the buffers fit, each
     // within kFrameStageMax and both within what the rest of the sign
     // kernel's shared memory leaves

@@ -119,18 +119,6 @@ __global__ void __launch_bounds__(32 * NW, 32 / NW) noise_vec_kernel(const Frame
     if (OWN && k >= w) return;
     const uint32_t *const s64 = J.slot_s64 + L.s64_base;
     const FrameSlotDev *const rec = J.slot + L.rec_base;
-    auto append = [&](bool hit, uint32_t slot, uint32_t u) {  // warp-aggregated; every lane calls it
-        const unsigned b = __ballot_sync(0xffffffffu, hit);
-        if (b == 0u) return;
-        uint32_t base = 0u;
-        if (lane == 0) base = atomicAdd(shit, (uint32_t)__popc(b));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (hit) {
-            const uint32_t at = base + __popc(b & ((1u << lane) - 1u));
-            shitl[2 * at] = slot;
-            shitl[2 * at + 1] = u;
-        }
-    };
     {
         const uint64_t e0 = rp.event_base + (uint64_t)L.ev0, g0 = e0 >> 2;
         const int64_t ngroups = (int64_t)(((e0 + (uint64_t)L.nslots - 1) >> 2) - g0 + 1);
@@ -154,15 +142,7 @@ __global__ void __launch_bounds__(32 * NW, 32 / NW) noise_vec_kernel(const Frame
             fetch(g + NT);
             const u32x4 blk =
                 draw_block(rp.seed, g0 + (uint64_t)g, rp.word_base + (uint64_t)k, 0u, TAG_NOISE_FIRST);
-            if (!OWN) {
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const int32_t sl = 4 * g + c + off0;
-                    append(sl >= 0 && sl < L.nslots && blk.v[c] >= now[c], (uint32_t)sl, blk.v[c]);
-                }
-                continue;
-            }
-            // one atomic for the four: here the chain of them is what counts
+            // the warp's hits of all four into the list, by one atomic
             uint32_t hit = 0u, all[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {

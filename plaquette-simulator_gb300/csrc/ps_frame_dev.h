@@ -157,19 +157,23 @@ inline int64_t noise_ctas(const FrameJobDev &j) {
     return ((int64_t)j.nnv * j.w + j.noise_units - 1) / j.noise_units;
 }
 // How many (range, shot-word) pairs a noise CTA takes, in a launch of `pairs`
-// of them.  The channels of a short range keep one warp busy, not four, and
-// its CTA is a chain of loads: where there are pairs enough to fill the chip
-// with six CTAs an SM, a warp each hides four times as much of it.  One kernel
-// per launch: a table whose jobs are not all short keeps a CTA a pair (a
-// kernel of both forms was 1 to 2 % slower at d = 15 and d = 21).  Measured, a
-// run with a CTA and with a warp a pair: d = 3, 60,000 shots, p = 5e-3 56 and
-// 47 us; d = 7, 30,000 shots, p = 1e-3 82 and 67; eight jobs up to d = 9 (430
-// channels a range) 170 and 133.
+// of them with at most `slots` channels each.  The channels of a short range
+// keep one warp busy, not four, and its CTA is a chain of loads: where there
+// are more pairs than six CTAs an SM take at once, a warp each hides four times
+// as much of it.  A longer range is a longer chain for its one warp, which
+// takes more pairs to hide.  One kernel per launch: a table whose jobs are not
+// all short keeps a CTA a pair (a kernel of both forms was 1 to 2 % slower at
+// d = 15 and d = 21).  Measured, a run with a CTA and with a warp a pair: d = 3,
+// 60,000 shots, p = 5e-3 55 and 45 us; d = 7, 15,000 and 30,000 shots, p = 1e-3
+// 46 and 41, 82 and 66; d = 9 (430 channels), p = 5e-3, 9,000 and 20,000 shots
+// 62 and 77, 96 and 98; eight jobs up to d = 9, to 27,000 shots 170 and 133;
+// fifteen, to 3,600 shots 61 and 77.
 constexpr uint32_t kNoiseWarpSlots = 512;
 constexpr int64_t kNoiseWarpPairs = 6 * 152;
-inline uint32_t noise_units(FrameJobDev j, int64_t pairs) {
+inline uint32_t noise_units(FrameJobDev j, int64_t pairs, uint32_t slots) {
     j.noise_units = kNoiseWarps;
-    return j.max_slots <= kNoiseWarpSlots && pairs > kNoiseWarpPairs && noise_job_smem(j) <= kNoiseSmemFloor ? kNoiseWarps : 1;
+    const bool many = pairs > kNoiseWarpPairs * std::max<int64_t>(160, slots) / 160;
+    return many && slots <= kNoiseWarpSlots && noise_job_smem(j) <= kNoiseSmemFloor ? kNoiseWarps : 1;
 }
 
 // One job of the x / z broadcast: X and Z of every (row, qubit) pair and

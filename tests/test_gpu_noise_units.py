@@ -1,5 +1,5 @@
 """Noise CTAs that take a (range, shot-word) pair a warp: launches with more
-than 912 pairs of at most 512 channels, against the per-shot kernels (which
+than 912 pairs (per 160 channels, of at most 512), against the per-shot kernels (which
 draw every channel by itself), alone and in a table of jobs; a last CTA with
 idle warps, and the sizes next to both limits."""
 import numpy as np
@@ -19,7 +19,8 @@ def _outputs(cc, st, circ):
 # warps); ranges of 500, 512 and 513 channels
 @pytest.mark.gpu
 @pytest.mark.parametrize("ranges,channels,shots", [(3, 50, 64 * 304), (3, 50, 64 * 306), (5, 7, 20001),
-                                                   (4, 500, 20000), (1, 512, 64 * 914), (1, 513, 64 * 914)])
+                                                   (4, 500, 46001), (1, 512, 64 * 2918), (1, 512, 64 * 2920),
+                                                   (1, 513, 64 * 2926)])
 def test_pairs_of_a_warp_equal_per_shot_kernels(ps, ranges, channels, shots):
     from plaquette_simulator import circuits as C
     from plaquette_simulator.circuit import CompiledCircuit
