@@ -383,8 +383,9 @@ def _stream_of(st, torch):
 
 def feed_forward_leg(args, shots, seed, torch, stream_of):
     """Circuits with per-shot feed-forward (H / S conditioned on each shot's
-    own measurement: the reference's ApplyFlag gates) take the per-shot
-    plan.  Workload: the batched low-space S-state distillation protocol
+    own measurement: the reference's ApplyFlag gates).  In this workload the
+    conditional gates are Paulis, so the fused form follows the shared x / z
+    on the device.  Workload: the batched low-space S-state distillation protocol
     (Test_CliffordState.hpp:675-741), --ff-blocks blocks of 5 qubits side by
     side, every shot of the headline's shot count.  Each step starts from
     |0...0>; the protocol's own check (data qubits 0..2 read 0, qubit 3
@@ -398,7 +399,7 @@ def feed_forward_leg(args, shots, seed, torch, stream_of):
     st = CliffordState(circ.num_qubits, shots, seed, True)
     stream = stream_of(st, torch)
     out = {"workload": f"S-state distillation, {args.ff_blocks} blocks of 5 qubits ({circ.num_qubits} qubits), "
-                       f"{shots} shots, per-shot plan (H_IF / S_IF feed-forward)",
+                       f"{shots} shots (H_IF / S_IF feed-forward)",
            "num_qubits": circ.num_qubits, "gates_per_shot": gates, "flag_gates_per_shot": flag,
            "measurements": circ.num_measurements(), "unit": "shot-gates/s"}
     for name, fused in (("fused", True), ("plain", False)):

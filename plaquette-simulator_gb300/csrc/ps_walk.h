@@ -7,7 +7,7 @@
 // are per shot.  From |0...0> the host knows the x / z and compiles a sign
 // program; the walk covers what it does not: runs without reset, whose
 // starting x / z are on the device only, and circuits with conditional
-// Paulis.  Four launches, whatever the circuit's length:
+// Paulis.  A few launches, whatever the circuit's length:
 //   gather     (runs without reset) reads the first shot's bits;
 //   check      (runs without reset, beside the walk; a small tableau's check
 //              is the gather's) reads X and Z once and checks that every (row, qubit) is the same in all shots; if

@@ -420,8 +420,8 @@ def distillation_blocks(blocks: int) -> Circuit:
     every block entangles its ancilla with the phasor's data qubits, rotates
     and measures it, then undoes the rotation on every qubit involved with
     H / S gates conditioned on that measurement (H_IF, S_IF: per-shot
-    feed-forward, so the circuit runs the per-shot plan).  The blocks step
-    through the phasors together, so each phasor's measurements form one
+    feed-forward; together they are conditional Paulis, so the shots keep
+    sharing their x / z and the run is a walk).  The blocks step through the phasors together, so each phasor's measurements form one
     measurement phase.  Afterwards data qubits 0..2 of every block measure
     0 and qubit 3 (after S, H) measures 1, all determined, in every shot."""
     c = Circuit(5 * blocks)
