@@ -253,6 +253,8 @@ struct ps_circuit {
     cudaEvent_t ev_ran = nullptr, ev_copied = nullptr;
     bool copy_pending = false;
     int32_t *h_err = nullptr;
+    int32_t *h_err_now = nullptr;  // the same for ps_circuit_copy_records
+    bool copied = false;
     // ps_circuit_detectors: its scratch, kept between calls (up to kDetKeep
     // bytes; not on a pooled state, whose pool others share).  Its three
     // allocations and frees were 25 us of a call.
@@ -2529,10 +2531,21 @@ ps_status ps_circuit_copy_records(ps_circuit *c, uint64_t *results, uint64_t *de
         PS_CUDA(cudaMemcpyAsync(results, c->d_res_block, bytes, cudaMemcpyDeviceToHost, h->stream));
     if (determined && bytes)
         PS_CUDA(cudaMemcpyAsync(determined, c->d_det_block, bytes, cudaMemcpyDeviceToHost, h->stream));
-    int32_t err = 0;  // the sign kernel's error word (shared-x/z runs)
-    if (c->d_ferr) PS_CUDA(cudaMemcpyAsync(&err, c->d_ferr, sizeof err, cudaMemcpyDeviceToHost, h->stream));
+    // The sign kernel's error word (shared-x/z runs), to pinned memory from the
+    // second call on: a copy to the stack waits for the stream by itself (3 us
+    // of a small call; the first call's circuit may never see another).
+    int32_t word = 0;
+    volatile int32_t *err = &word;
+    if (c->d_ferr && c->copied && !c->h_err_now && cudaMallocHost(&c->h_err_now, sizeof(int32_t)) != cudaSuccess) {
+        cudaGetLastError();
+        c->h_err_now = nullptr;
+    }
+    c->copied = true;
+    if (c->h_err_now) err = c->h_err_now;
+    if (c->d_ferr)
+        PS_CUDA(cudaMemcpyAsync(const_cast<int32_t *>(err), c->d_ferr, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
     PS_CUDA(cudaStreamSynchronize(h->stream));
-    if (err) return fail(E_TIMEOUT, "a copy of the sign program did not arrive in time; the run's records are void");
+    if (*err) return fail(E_TIMEOUT, "a copy of the sign program did not arrive in time; the run's records are void");
     return OK;
 }
 
@@ -2692,6 +2705,7 @@ ps_status ps_circuit_destroy(ps_circuit *c) {
     if (c->ev_ran) cudaEventDestroy(c->ev_ran);
     if (c->ev_copied) cudaEventDestroy(c->ev_copied);
     if (c->h_err) cudaFreeHost(c->h_err);
+    if (c->h_err_now) cudaFreeHost(c->h_err_now);
     for (void *p : c->owned) dev_free(c->h, p);
     dev_free(c->h, c->d_forced);
     dev_free(c->h, c->d_det_scratch);

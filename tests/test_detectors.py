@@ -85,3 +85,22 @@ def test_detector_definitions_of_any_size(ps, shots, ndet, nidx):
     for some in (defs[:1], defs, defs[-2:]):
         want = np.stack([np.bitwise_xor.reduce(res[d], axis=0) if d else np.zeros_like(res[0]) for d in some])
         assert np.array_equal(cc.detectors(some), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shots", [64, 200])
+def test_record_copies_of_runs_in_turn(ps, shots):
+    """The first and later copies of a circuit's records (the later ones with
+    the error word in pinned memory) against the records one by one."""
+    from plaquette_simulator import circuits as C
+    from plaquette_simulator.circuit import CompiledCircuit
+    circ = C.surface_code_memory(3, 2, p=2e-2)
+    st = ps.CliffordState(circ.num_qubits, shots, 6, True)
+    cc = CompiledCircuit(circ, st)
+    nm = circ.num_measurements()
+    for _ in range(3):
+        cc.run(reset=True)
+        res = np.zeros((nm, ((shots + 63) // 64 + 1) & ~1), np.uint64)
+        cc.copy_records_words(res, None)
+        want, _ = cc.records()
+        assert np.array_equal(_bits(res, shots), want)
